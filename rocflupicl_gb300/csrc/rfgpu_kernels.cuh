@@ -14,6 +14,7 @@
 #pragma once
 
 #include "rfgpu_internal.h"
+#include "rfgpu_soft64.cuh"
 
 namespace rfgpu {
 
@@ -986,6 +987,213 @@ __device__ __forceinline__ double cell_dt(const RegionDev<R> &g, int c, const R 
 #ifndef RF_GRAD_MINB_DT
 #define RF_GRAD_MINB_DT 8  // the same for the stage-1 pass that also reduces the time step
 #endif
+// ---- FP64 gradient pass ------------------------------------------------------------
+// Bound by the FP64 pipe (one warp operation per 64 cycles and SM quarter), so
+// the pass keeps off it what has an exact equivalent elsewhere: the products
+// of the member sum and of the limiter's d2 are integer products (soft_mul,
+// the same bits), the min / max comparisons run on the bit patterns, and the
+// limiter's quotients are first formed in FP32 to find the face that decides
+// each variable's minimum, whose quotient alone is then formed in FP64.
+// FP64 operations per tet cell with 40 members: about 980 against 2440.
+
+// b < a for numbers that are neither infinite nor NaN.  (-0 counts as below
+// +0; a zero's sign never reaches the limiter's result.)
+__device__ __forceinline__ bool lt_bits(double b, double a) {
+  long long kb = __double_as_longlong(b), ka = __double_as_longlong(a);
+  kb ^= (kb >> 63) & 0x7fffffffffffffffll;
+  ka ^= (ka >> 63) & 0x7fffffffffffffffll;
+  return kb < ka;
+}
+__device__ __forceinline__ bool finite_bits(double x) {
+  return ((unsigned)__double2hiint(x) & 0x7ff00000u) != 0x7ff00000u;
+}
+// FP32 value of a double of magnitude in [2^-100, 2^40) (truncated); other
+// values, zero apart, clear ok.
+__device__ __forceinline__ float narrow_bits(double x, bool &ok) {
+  const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
+  const unsigned t = h & 0x7fffffffu;
+  if ((t | l) == 0u) return 0.f;
+  ok = ok && t - (923u << 20) < (140u << 20);
+  return __uint_as_float((h & 0x80000000u) | __funnelshift_l(l, t - (896u << 20), 3));
+}
+
+// Screening of one variable's Venkatakrishnan terms.  In FP32 a term's
+// numerator and denominator are sums of terms of one sign (d2 and its bound dm
+// have the same sign), so its relative error stays below 3e-6 when nothing
+// leaves FP32's normal range; two terms further apart than 1e-5 are then
+// ordered as in FP64, and only the smallest one decides the limiter.  What the
+// screen cannot order - two different d2 within 1e-5, magnitudes outside the
+// ranges below, the reference's cancelling guard - is left to the FP64 loop.
+struct VenkatScreen {
+  float best, second;
+  double d2;  // of the smallest term
+};
+__device__ __forceinline__ void venkat_screen(VenkatScreen &s, double d2, float mx, float mn,
+                                              float e, int guard, bool &ok) {
+  const float x = narrow_bits(d2, ok);
+  if (soft_zero(d2)) return;  // the reference skips d2 = 0
+  const bool pos = x > 0.f;
+  const float m = pos ? mx : mn;
+  const float a = fmaf(m, m, e), xm = x * m;
+  const float num = x * fmaf(2.f, xm, a);
+  const float den0 = x * (fmaf(2.f * x, x, a) + xm), mag = fabsf(den0);
+  ok = ok && mag > 1e-30f && mag < 1e30f && (pos || guard || mag > 1e-6f);
+  const float t = __fdividef(num, den0 + ((pos || !guard) ? 1e-12f : -1e-12f));
+  if (__double_as_longlong(d2) != __double_as_longlong(s.d2)) {  // an equal d2 has an equal term
+    s.second = fminf(s.second, fmaxf(s.best, t));
+    if (t < s.best) {
+      s.best = t;
+      s.d2 = d2;
+    }
+  }
+}
+
+// One variable v of one cell of the FP64 gradient pass.  Every sum and rounding
+// is the reference's, in its order.  Returns the cell's local time step bits
+// (FUSE_DT, first variable only).  RF_G64_U members' loads are issued ahead of
+// their sums (64^3 tet box: 1 -> 3.26 ms, 2 -> 3.24, 4 -> 3.34).
+#ifndef RF_G64_U
+#define RF_G64_U 2
+#endif
+template <int FUSE_DT>
+__device__ __forceinline__ unsigned long long grad_cell64(const RegionDev<double> &g, int c,
+                                                          int v) {
+  const double *__restrict__ rec = g.rec + v;
+  const bool withDt = FUSE_DT && v == 0;
+  unsigned long long dtbits = 0x7FF0000000000000ull;
+  const double r0 = rec[8 * (size_t)c];
+  const long long e0 = g.cfOff[c >> 5] + (c & 31);
+  const int nf = g.cfCnt[c];
+  double acc[3] = {0.0, 0.0, 0.0};
+  {
+    constexpr int U = RF_G64_U;
+    const int n = g.stCnt[c];
+    const long long base = g.stOff[c >> 5] + (c & 31), T = g.stTotal;
+    const int *__restrict__ sidx = g.stIdx + base;
+    const double *__restrict__ w0 = g.stW + base;
+    auto member = [&](double q, const double w[3]) {
+      q = q - r0;
+      if (soft_ok(q) && soft_ok(w[0]) && soft_ok(w[1]) && soft_ok(w[2])) {
+        const SoftB b = soft_b(q);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) acc[d] = acc[d] + soft_mul(soft_a(w[d]), b);
+      } else {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) acc[d] = acc[d] + w[d] * q;
+      }
+    };
+    int nx[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) nx[u] = u < n ? sidx[u * kSlice] : 0;
+    for (int k = 0; k < n; k += U) {
+      double q[U], w[U][3];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        q[u] = rec[8 * (size_t)nx[u]];
+        const int kk = k + u < n ? k + u : k;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) w[u][d] = w0[d * T + kk * kSlice];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) nx[u] = k + U + u < n ? sidx[(k + U + u) * kSlice] : 0;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u == 0 || k + u < n) member(q[u], w[u]);
+    }
+  }
+  if (g.ph.reconst == 11) {
+    double vmin = r0, vmax = r0;
+    const long long T = g.cfTotal;
+    double dtacc = 0.0, a0 = 0.0, rc[8];
+    if (withDt) {
+      ld8(g.rec + 8 * (size_t)c, rc);
+      a0 = dt_sound(g, c, rc);
+    }
+    const bool fin0 = finite_bits(r0);
+    for (int k = 0; k < nf; ++k) {
+      const long long ee = e0 + (long long)k * kSlice;
+      const int code = g.cfCode[ee];
+      if (code < 0) {
+        if (withDt) dt_boundary_term(g, code, rc, a0, dtacc);
+        continue;
+      }
+      const int nb = g.cfNb[ee];
+      const double q = rec[8 * (size_t)nb];
+      if (fin0 && finite_bits(q)) {
+        if (lt_bits(q, vmin)) vmin = q;
+        if (lt_bits(vmax, q)) vmax = q;
+      } else {
+        vmin = rmin(vmin, q);
+        vmax = rmax(vmax, q);
+      }
+      if (withDt) {
+        double rn[8];
+        ld8(g.rec + 8 * (size_t)nb, rn);
+        dt_interior_term(g, code, rc, a0, nb, rn, dtacc);
+      }
+    }
+    if (withDt) {
+      dtbits = (unsigned long long)__double_as_longlong(dt_of(g, c, dtacc));
+      if (c >= g.nAct) dtbits = 0x7FF0000000000000ull;  // actual cells only
+    }
+    const double epsq = g.epsq[c];
+    const int guard = g.ph.venkatGuard;
+    vmax = vmax - r0;  // the bounds dmax, dmin
+    vmin = vmin - r0;
+    bool ok = epsq > 1e-25 && epsq < 1e12;
+    const float ef = ok ? (float)epsq : 1.f;
+    const float mx = narrow_bits(vmax, ok), mn = narrow_bits(vmin, ok);
+    ok = ok && soft_ok(acc[0]) && soft_ok(acc[1]) && soft_ok(acc[2]);
+    const SoftB bx = soft_b(acc[0]), by = soft_b(acc[1]), bz = soft_b(acc[2]);
+    VenkatScreen sc = {3.0e38f, 3.0e38f, 0.0};
+    for (int k = 0; k < nf; ++k) {
+      const long long ee = e0 + (long long)k * kSlice;
+      if (g.cfCode[ee] < 0) continue;
+      const double dx = g.cfD[ee], dy = g.cfD[T + ee], dz = g.cfD[2 * T + ee];
+      ok = ok && soft_ok(dx) && soft_ok(dy) && soft_ok(dz);
+      if (ok) {
+        const double d2 =
+            soft_mul(soft_a(dx), bx) + soft_mul(soft_a(dy), by) + soft_mul(soft_a(dz), bz);
+        venkat_screen(sc, d2, mx, mn, ef, guard, ok);
+      }
+    }
+    double lim = 1.0;
+    const float near = 1.00001f;
+    if (ok && !(sc.best <= near && sc.second <= sc.best * near)) {
+      if (sc.best <= near) venkat_term(sc.d2, vmax, vmin, epsq, lim, guard);
+    } else {
+      for (int k = 0; k < nf; ++k) {
+        const long long ee = e0 + (long long)k * kSlice;
+        if (g.cfCode[ee] < 0) continue;
+        const double d2 = acc[0] * g.cfD[ee] + acc[1] * g.cfD[T + ee] + acc[2] * g.cfD[2 * T + ee];
+        venkat_term(d2, vmax, vmin, epsq, lim, guard);
+      }
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) acc[d] = lim * acc[d];
+  }
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    if (!g.gradRaw) {
+      g.grad[16 * (size_t)c + 3 * v + d] = acc[d];
+    } else {
+      // RECONST 2: the WENO weight of each component and its product, as
+      // RFLU_WENOGradCellsXYZFast_3D forms them (same operations), once per
+      // cell instead of once per stencil visit
+      const double w = 1.0 / (acc[d] * acc[d] + 1.0E-15);
+      g.gradRaw[32 * (size_t)c + 3 * v + d] = w;
+      g.gradRaw[32 * (size_t)c + 16 + 3 * v + d] = w * acc[d];
+    }
+  }
+  if (withDt && g.ph.reconst != 11) {  // no limiter face loop to ride on
+    double rc[8];
+    ld8(g.rec + 8 * (size_t)c, rc);
+    dtbits = (unsigned long long)__double_as_longlong(cell_dt(g, c, rc));
+    if (c >= g.nAct) dtbits = 0x7FF0000000000000ull;
+  }
+  return dtbits;
+}
+
 // BS threads per block (one cell each, a tile of BS cells); the requested
 // residency keeps the same number of resident threads per SM for every BS.
 // One tile of the gradient pass (every thread of the block, one cell each).
@@ -1006,7 +1214,12 @@ __device__ __forceinline__ void grad_tile(const RegionDev<R> *__restrict__ regs,
     const long long base = valid ? g.stOff[c >> 5] + (c & 31) : 0;
     const int *__restrict__ sidx = g.stIdx + base;
     unsigned long long dtbits = 0x7FF0000000000000ull;
-    if (valid) {
+    if constexpr (sizeof(R) == 8) {
+      if (valid) {  // the persistent stage kernel: a thread takes a cell's variables in turn
+        dtbits = grad_cell64<FUSE_DT>(g, c, 0);
+        for (int v = 1; v < 5; ++v) grad_cell64<0>(g, c, v);
+      }
+    } else if (valid) {
       const R *__restrict__ rec = g.rec;
       R r0[8];
       ld8(rec + 8 * (size_t)c, r0);
@@ -1014,34 +1227,7 @@ __device__ __forceinline__ void grad_tile(const RegionDev<R> *__restrict__ regs,
 #pragma unroll
       for (int k = 0; k < 15; ++k) acc[k] = R(0);
       const int n = g.stCnt[c];
-      // members accumulated in stored order; loads of consecutive members are
-      // issued together so their gathers overlap
-      if (sizeof(R) == 8) {
-        const long long T = g.stTotal;
-        auto member = [&](const R rn[8], long long ee) {
-          const R wx = g.stW[ee], wy = g.stW[T + ee], wz = g.stW[2 * T + ee];
-#pragma unroll
-          for (int v = 0; v < 5; ++v) {
-            R dVar = rn[v] - r0[v];
-            acc[3 * v] = acc[3 * v] + wx * dVar;
-            acc[3 * v + 1] = acc[3 * v + 1] + wy * dVar;
-            acc[3 * v + 2] = acc[3 * v + 2] + wz * dVar;
-          }
-        };
-        int k = 0;
-        for (; k + 2 <= n; k += 2) {
-          R ra[8], rb[8];
-          ld8(rec + 8 * (size_t)sidx[k * kSlice], ra);
-          ld8(rec + 8 * (size_t)sidx[(k + 1) * kSlice], rb);
-          member(ra, base + (long long)k * kSlice);
-          member(rb, base + (long long)(k + 1) * kSlice);
-        }
-        for (; k < n; ++k) {
-          R ra[8];
-          ld8(rec + 8 * (size_t)sidx[k * kSlice], ra);
-          member(ra, base + (long long)k * kSlice);
-        }
-      } else {
+      {
         // The reference's weight of member m is w = A d/|d|^2 with d the
         // centroid offset and A the cell's symmetric inverse-moment matrix
         // built from its WLSQ factor (c11^2 + c12^2 c22^2 + c13^2 c33^2, ...).
@@ -1178,18 +1364,6 @@ __device__ __forceinline__ void grad_tile(const RegionDev<R> *__restrict__ regs,
       out[15] = R(0);
       if (!g.gradRaw) {
         st16(g.grad + 16 * (size_t)c, out);
-      } else if constexpr (sizeof(R) == 8) {
-        // RECONST 2, FP64: the WENO weight of each component and its product,
-        // as RFLU_WENOGradCellsXYZFast_3D forms them (same operations), once
-        // per cell instead of once per stencil visit
-        R w[16];
-#pragma unroll
-        for (int k = 0; k < 15; ++k) w[k] = R(1) / (out[k] * out[k] + R(1.0E-15));
-        w[15] = R(0);
-        st16(g.gradRaw + 32 * (size_t)c, w);
-#pragma unroll
-        for (int k = 0; k < 15; ++k) w[k] = w[k] * out[k];
-        st16(g.gradRaw + 32 * (size_t)c + 16, w);
       } else {
         st16(g.gradRaw + 16 * (size_t)c, out);  // RECONST 2, mixed: weighted next
       }
@@ -1201,6 +1375,41 @@ __device__ __forceinline__ void grad_tile(const RegionDev<R> *__restrict__ regs,
       }
     }
     if constexpr (fuseDt) dt_block_min<R>(dtbits, smin, g.dtBits);
+  }
+}
+
+// FP64: one warp per 32 cells and variable, so that a region of a few thousand
+// cells reaches every SM quarter's FP64 unit and a large one needs 80 registers
+// a thread instead of 128.  Measured (pass with its launch): 512 cells 48.8 ->
+// 22.8 us, 4,000 cells 49.0 -> 22.9, 64,000 cells 98 -> 66, 1.57 M cells 6.08
+// -> 3.24 ms, about 975 FP64 operations per cell at 0.51 T/s (one thread per
+// cell with all five variables: 67 us, 67 us, 84 us, 3.28 ms).  Residency
+// asked for on 1.57 M cells: 4 blocks 3.63 ms, 5 3.26, 6 3.24, 7 3.21 (2 to 5%
+// slower below 20,000 cells).
+// The five warps of 32 cells form a block (blockDim.y = 5) and share the
+// weights in L1 where there are slices enough to level the SM quarters out
+// (kGrad64Rows; at 64,000 cells 67 against 64 us, the same from 235,000 on);
+// otherwise they are five blocks (gridDim.y = 5).  per = 32-cell slices of a
+// tile.
+constexpr int kGrad64Rows = 4000;
+template <int FUSE_DT>
+__global__ void __launch_bounds__(160, 6)
+    k_grad_lim64(const RegionDev<double> *__restrict__ regs, const Tile *__restrict__ tiles,
+                 int nTiles, int per) {
+  const int v = blockIdx.y * blockDim.y + threadIdx.y;
+  for (int i = blockIdx.x; i < nTiles * per; i += gridDim.x) {
+    const Tile tl = tiles[i / per];
+    const RegionDev<double> &g = regs[tl.region];
+    const int c = tl.first + i % per * 32 + (int)threadIdx.x;
+    unsigned long long bits = 0x7FF0000000000000ull;
+    if (c < g.nCells) bits = grad_cell64<FUSE_DT>(g, c, v);
+    if (FUSE_DT && v == 0) {
+      for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long x = __shfl_down_sync(0xffffffffu, bits, o);
+        bits = x < bits ? x : bits;
+      }
+      if (threadIdx.x == 0 && bits < __ldcg(g.dtBits)) atomicMin(g.dtBits, bits);
+    }
   }
 }
 
@@ -2379,8 +2588,18 @@ inline int grid_for(int cap, int nTiles) { return cap > 0 && cap < nTiles ? cap 
 
 template <typename R, int F, int BS>
 void grad_launch(const RegionDev<R> *regs, const Tile *tiles, int nTiles, int cap, cudaStream_t s) {
+  if constexpr (sizeof(R) == 8) {
+    const int per = BS / 32, n = grid_for(cap, nTiles * per);
+    if (n <= 0) return;
+    if (n == nTiles * per && n < kGrad64Rows)
+      k_grad_lim64<F><<<dim3(n, 5), dim3(32, 1), 0, s>>>(regs, tiles, nTiles, per);
+    else
+      k_grad_lim64<F><<<n, dim3(32, 5), 0, s>>>(regs, tiles, nTiles, per);
+    return;
+  }
   const int grid = grid_for(cap, nTiles);
-  if (grid > 0) k_grad_lim<R, F, BS><<<grid, BS, 0, s>>>(regs, tiles, nTiles);
+  if constexpr (sizeof(R) == 4)
+    if (grid > 0) k_grad_lim<R, F, BS><<<grid, BS, 0, s>>>(regs, tiles, nTiles);
 }
 
 template <typename R>
