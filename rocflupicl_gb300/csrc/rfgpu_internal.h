@@ -7,6 +7,8 @@
 // (mixed path) instead of one per component:
 //   cell state   cv[5][N], rhsSum[5][N], dv[3][N] (p,T,a)        FP64 SoA
 //   cell record  rec[N][8] = rho,u,v,w,p,x,y,z                   R    AoS
+//                (FP64 path: the face loops' starting velocities in place of
+//                x,y,z, whose weights are precomputed there)
 //   gradients    grad[N][16] = d(rho,u,v,w,p)/d(x,y,z)           R    AoS
 //   stencil      SELL-32: member k of cell c at stOff[c/32] + 32*k + c%32;
 //                stIdx (0-based); stW[3][stTotal] precomputed WLSQ weights
@@ -70,7 +72,8 @@ struct RegionDev {
   double *cv, *cvOld, *rhsSum, *dv, *rhs;
   float *rhsSumF;
   float *cvF, *cvOldF;
-  // gathered per-cell records (AoS): rec[8*c..] = rho,u,v,w,p,x,y,z;
+  // gathered per-cell records (AoS): rec[8*c..] = rho,u,v,w,p,x,y,z (FP64
+  // path: slots 5..7 hold the velocities of cell_values);
   // grad[16*c + 3*v + d] (15 used)
   R *rec, *grad;
   // geometry

@@ -71,4 +71,48 @@ __device__ __forceinline__ double soft_mul(const SoftA &a, const SoftB &b) {
   return __hiloint2double((int)(r1 & a.z & b.z), (int)r0);
 }
 
+// A double for arithmetic written over a number type, whose products are
+// FP64 operations as usual unless asked for as prod(), an integer product, or
+// scale<K>(), a product with 2^K done on the exponent.  An operand outside
+// their range makes the result NaN instead of taking a branch; NaN reaches
+// every result that depends on it, and the caller repeats such a rare
+// evaluation on plain doubles.  Comparisons do not hide it: minimum, maximum
+// and positive part keep NaN, and `unknown` tells that a branch condition is
+// NaN (for plain numbers it is false at compile time, their NaNs being
+// results).
+struct Sd {
+  double v;
+  __device__ __forceinline__ Sd() {}
+  __device__ __forceinline__ constexpr explicit Sd(double x) : v(x) {}
+  friend __device__ __forceinline__ Sd sqrt(Sd a) { return Sd(::sqrt(a.v)); }
+  friend __device__ __forceinline__ Sd fabs(Sd a) { return Sd(::fabs(a.v)); }
+};
+__device__ __forceinline__ Sd operator+(Sd a, Sd b) { return Sd(a.v + b.v); }
+__device__ __forceinline__ Sd operator-(Sd a, Sd b) { return Sd(a.v - b.v); }
+__device__ __forceinline__ Sd operator-(Sd a) { return Sd(-a.v); }
+__device__ __forceinline__ Sd operator/(Sd a, Sd b) { return Sd(a.v / b.v); }
+__device__ __forceinline__ Sd operator*(Sd a, Sd b) { return Sd(a.v * b.v); }
+template <typename R> __device__ __forceinline__ R prod(R a, R b) { return a * b; }
+template <> __device__ __forceinline__ Sd prod(Sd a, Sd b) {
+  const double r = soft_mul(soft_a(a.v), soft_b(b.v));
+  const unsigned bad = (soft_ok(a.v) ? 0u : 0x7ff80000u) | (soft_ok(b.v) ? 0u : 0x7ff80000u);
+  return Sd(__hiloint2double((int)((unsigned)__double2hiint(r) | bad), __double2loint(r)));
+}
+constexpr double pow2(int k) { return k == 0 ? 1.0 : k > 0 ? 2.0 * pow2(k - 1) : 0.5 * pow2(k + 1); }
+template <int K, typename R> __device__ __forceinline__ R scale(R x) { return R(pow2(K)) * x; }
+template <int K> __device__ __forceinline__ Sd scale(Sd x) {
+  const unsigned h = (unsigned)__double2hiint(x.v), l = (unsigned)__double2loint(x.v);
+  const bool ok = (h & 0x7fffffffu) - 0x01000000u < 0x7e000000u;  // exponents 16 .. 2031
+  const unsigned r = ok ? h + (unsigned)(K * (1 << 20)) : soft_zero(x.v) ? h : 0x7ff80000u;
+  return Sd(__hiloint2double((int)r, (int)l));
+}
+__device__ __forceinline__ bool operator<(Sd a, Sd b) { return a.v < b.v; }
+__device__ __forceinline__ bool operator>(Sd a, Sd b) { return a.v > b.v; }
+__device__ __forceinline__ bool operator<=(Sd a, Sd b) { return a.v <= b.v; }
+__device__ __forceinline__ bool nan_bits(double x) {
+  const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+  return h > 0x7ff00000u || (h == 0x7ff00000u && __double2loint(x) != 0);
+}
+__device__ __forceinline__ bool unknown(Sd a) { return nan_bits(a.v); }
+
 }  // namespace rfgpu
