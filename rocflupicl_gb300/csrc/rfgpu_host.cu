@@ -1357,6 +1357,7 @@ int rfgpu_region_create(const rfgpu_region_desc_t *d, rfgpu_region_t *out) {
     h->work.split = h->prec == RFGPU_PREC_SPLIT;
     h->work.bar = h->mem.alloc<GridBar>(1);
     h->work.barSpin = kBarrierSpin;
+    h->work.one = h->prec ? (const void *)&h->rd32 : (const void *)&h->rd64;
     cudaMemsetAsync(h->work.bar, 0, sizeof(GridBar), h->stream);
     h->stage = h->mem.alloc<double>(5 * (size_t)h->nCells);
     if (h->prec) h->stage2 = h->mem.alloc<double>(3 * (size_t)h->nCells);

@@ -181,6 +181,9 @@ struct Work {
   // runs out) and the wait's limit in SM clock cycles
   int barExtra;
   long long barSpin;
+  // a single region's descriptor on the host (RegionDev of the kernels'
+  // precision), or null: launches pass it by value instead of the table
+  const void *one;
 };
 
 struct DtArgs {

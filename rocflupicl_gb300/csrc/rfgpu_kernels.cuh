@@ -13,6 +13,8 @@
 // count walk the list persistently.
 #pragma once
 
+#include <type_traits>
+
 #include "rfgpu_internal.h"
 #include "rfgpu_soft64.cuh"
 
@@ -660,6 +662,29 @@ __device__ __forceinline__ int pdl_wait() {
 #define RF_TILE_LOOP(first, nTiles) \
   for (int t_ = (first); t_ < (nTiles); t_ += gridDim.x)
 
+// Where a kernel finds its regions: a device table (batches), or, for a single
+// region, its descriptor as a kernel parameter.  The descriptor's fields are
+// then constant-bank operands instead of loads and of registers that hold
+// them, and without a tile list (its tiles are consecutive) the two dependent
+// loads of tile and descriptor ahead of a tile's own are gone.  Measured, mixed:
+// 12.6 M tets gradient 1.72 -> 1.57 ms (20 bytes of spills gone), faces 0.628
+// -> 0.548, WENO pass of 1.57 M tets 0.424 -> 0.396, a step of 10,000 tets 67.7
+// -> 61.6 us.  FP64, bound by its pipe, gains 1 to 3%.
+template <typename R> struct OneRegion {
+  RegionDev<R> r;
+  __device__ __forceinline__ const RegionDev<R> &operator[](int) const { return r; }
+};
+template <typename R>
+__device__ __forceinline__ Tile tile_at(const RegionDev<R> *, const Tile *__restrict__ tiles, int t,
+                                        int) {
+  return tiles[t];
+}
+template <typename R>
+__device__ __forceinline__ Tile tile_at(const OneRegion<R> &, const Tile *__restrict__ tiles, int t,
+                                        int stride) {
+  return tiles ? tiles[t] : Tile{0, t * stride};
+}
+
 // Cons2Prim (modflu/RFLU_ModConvertCv.F90:221-231) of one cell's FP64 state
 // into its record, and optionally the EOS first (libflu/RFLU_SetDependentVars.F90:
 // 256-287).  The record's centroid slots are kept.  FP64 path.
@@ -1257,13 +1282,12 @@ __device__ __forceinline__ unsigned long long grad_cell64(const RegionDev<double
 // BS threads per block (one cell each, a tile of BS cells); the requested
 // residency keeps the same number of resident threads per SM for every BS.
 // One tile of the gradient pass (every thread of the block, one cell each).
-template <typename R, int FUSE_DT>
-__device__ __forceinline__ void grad_tile(const RegionDev<R> *__restrict__ regs,
-                                          const Tile *__restrict__ tiles, int t_,
+template <typename R, int FUSE_DT, typename RT>
+__device__ __forceinline__ void grad_tile(const RT &regs, const Tile *__restrict__ tiles, int t_,
                                           unsigned long long *smin) {
   constexpr bool fuseDt = FUSE_DT != 0;
   {
-    const Tile tl = tiles[t_];
+    const Tile tl = tile_at(regs, tiles, t_, blockDim.x);
     const RegionDev<R> &g = regs[tl.region];
     const int c = tl.first + threadIdx.x;
     const int N = g.nCells;
@@ -1430,7 +1454,7 @@ __device__ __forceinline__ void grad_tile(const RegionDev<R> *__restrict__ regs,
       if constexpr (fuseDt) {
         if (g.ph.reconst != 11) {  // no limiter face loop to ride on
           dtbits = (unsigned long long)__double_as_longlong(cell_dt(g, c, r0));
-          if (c >= regs[tl.region].nAct) dtbits = 0x7FF0000000000000ull;
+          if (c >= g.nAct) dtbits = 0x7FF0000000000000ull;
         }
       }
     }
@@ -1452,13 +1476,12 @@ __device__ __forceinline__ void grad_tile(const RegionDev<R> *__restrict__ regs,
 // otherwise they are five blocks (gridDim.y = 5).  per = 32-cell slices of a
 // tile.
 constexpr int kGrad64Rows = 4000;
-template <int FUSE_DT>
-__global__ void __launch_bounds__(160, 6)
-    k_grad_lim64(const RegionDev<double> *__restrict__ regs, const Tile *__restrict__ tiles,
-                 int nTiles, int per) {
+template <int FUSE_DT, typename RT>
+__device__ __forceinline__ void grad64_body(const RT &regs, const Tile *__restrict__ tiles,
+                                            int nTiles, int per) {
   const int v = blockIdx.y * blockDim.y + threadIdx.y;
   for (int i = pdl_wait(); i < nTiles * per; i += gridDim.x) {
-    const Tile tl = tiles[i / per];
+    const Tile tl = tile_at(regs, tiles, i / per, per * 32);
     const RegionDev<double> &g = regs[tl.region];
     const int c = tl.first + i % per * 32 + (int)threadIdx.x;
     unsigned long long bits = 0x7FF0000000000000ull;
@@ -1472,11 +1495,30 @@ __global__ void __launch_bounds__(160, 6)
     }
   }
 }
+template <int FUSE_DT>
+__global__ void __launch_bounds__(160, 6)
+    k_grad_lim64(const RegionDev<double> *__restrict__ regs, const Tile *__restrict__ tiles,
+                 int nTiles, int per) {
+  grad64_body<FUSE_DT>(regs, tiles, nTiles, per);
+}
+template <int FUSE_DT>
+__global__ void __launch_bounds__(160, 6)
+    k_grad_lim64(const __grid_constant__ OneRegion<double> regs, const Tile *__restrict__ tiles,
+                 int nTiles, int per) {
+  grad64_body<FUSE_DT>(regs, tiles, nTiles, per);
+}
 
 template <typename R, int FUSE_DT, int BS>
 __global__ void __launch_bounds__(BS, ((sizeof(R) == 4) ? (FUSE_DT ? RF_GRAD_MINB_DT : RF_GRAD_MINB)
                                                         : 4) * 128 / BS)
     k_grad_lim(const RegionDev<R> *__restrict__ regs, const Tile *__restrict__ tiles, int nTiles) {
+  __shared__ unsigned long long smin[32];
+  RF_TILE_LOOP(pdl_wait(), nTiles) grad_tile<R, FUSE_DT>(regs, tiles, t_, smin);
+}
+template <typename R, int FUSE_DT, int BS>
+__global__ void __launch_bounds__(BS, ((sizeof(R) == 4) ? (FUSE_DT ? RF_GRAD_MINB_DT : RF_GRAD_MINB)
+                                                        : 4) * 128 / BS)
+    k_grad_lim(const __grid_constant__ OneRegion<R> regs, const Tile *__restrict__ tiles, int nTiles) {
   __shared__ unsigned long long smin[32];
   RF_TILE_LOOP(pdl_wait(), nTiles) grad_tile<R, FUSE_DT>(regs, tiles, t_, smin);
 }
@@ -1605,14 +1647,13 @@ __device__ __forceinline__ void face_flux_one(const RegionDev<R> &g, int f) {
   }
 }
 
-template <typename R, int BS, int FPT>
-__device__ __forceinline__ void face_tile(const RegionDev<R> *__restrict__ regs,
-                                          const Tile *__restrict__ tiles, int nTiles, int t_,
-                                          int dist) {
-  const Tile tl = tiles[t_];
+template <typename R, int BS, int FPT, typename RT>
+__device__ __forceinline__ void face_tile(const RT &regs, const Tile *__restrict__ tiles,
+                                          int nTiles, int t_, int dist) {
+  const Tile tl = tile_at(regs, tiles, t_, BS * FPT);
   const RegionDev<R> &g = regs[tl.region];
   prefetch_ahead(t_, nTiles, dist, [&](int t) {
-    const Tile tp = tiles[t];
+    const Tile tp = tile_at(regs, tiles, t, BS * FPT);
     prefetch_face_tile(regs[tp.region], tp.first, BS * FPT);
   });
 #pragma unroll
@@ -1661,8 +1702,8 @@ __device__ __forceinline__ void dt_finalize_region(const RegionDev<R> &g, unsign
 // to the minimum gives the reference's minimum of the per-region results.  The
 // raw minima are read through L2: in the persistent stage kernel other blocks
 // reduced them earlier in the same launch.
-template <typename R>
-__device__ __forceinline__ void dt_finalize_block(const RegionDev<R> *__restrict__ regs,
+template <typename R, typename RT>
+__device__ __forceinline__ void dt_finalize_block(const RT &regs,
                                                   int nRegions, int coupled,
                                                   const DtArgs &a, unsigned long long *smin) {
   if (!coupled) {
@@ -1852,11 +1893,10 @@ __device__ __forceinline__ void bcond_outflow(int bcOpt, R pout, R sxn, R syn, R
 // as mass flux, the exact additive identity, since the reference leaves the
 // mass residual untouched there.
 constexpr int kBTile = 128;  // boundary faces per tile, whatever the block size
-template <typename R>
-__device__ __forceinline__ void bface_tile(const RegionDev<R> *__restrict__ regs,
-                                           const Tile *__restrict__ tiles, int t_) {
+template <typename R, typename RT>
+__device__ __forceinline__ void bface_tile(const RT &regs, const Tile *__restrict__ tiles, int t_) {
   {
-    const Tile tl = tiles[t_];
+    const Tile tl = tile_at(regs, tiles, t_, kBTile);
     const RegionDev<R> &g = regs[tl.region];
     const int B = g.nBFaces;
     const int last = tl.first + kBTile < B ? tl.first + kBTile : B;
@@ -2000,17 +2040,53 @@ struct FluxExtra {
   DtArgs a;
 };
 
-// FP64: bound by the FP64 pipe; 128 registers asked for (168: the same time,
-// 102: 1% slower).  64^3 tets AUSM+ 1.53 -> 1.11 ms, AUSM+up 1.76 -> 1.32,
-// Roe 2.42 -> 1.83, HLLC 1.82 -> 1.44 with the reconstruction and prod()
-// products on the integer pipes (the reconstruction alone: 1.32, 1.54, 2.14,
-// 1.60), the exponent scalings, and the velocities kept per cell.
 template <typename R, int BS, int FPT>
-__global__ void __launch_bounds__(BS, (sizeof(R) == 4 ? 0 : 4 * 128 / BS))
+__global__ void __launch_bounds__(BS)
     k_face_flux(const RegionDev<R> *__restrict__ regs, const Tile *__restrict__ tiles, int nTiles,
                 int pfDist) {
   const int dist = (int)gridDim.x < nTiles ? (int)gridDim.x : pfDist;
   RF_TILE_LOOP(pdl_wait(), nTiles) face_tile<R, BS, FPT>(regs, tiles, nTiles, t_, dist);
+}
+template <typename R, int BS, int FPT>
+__global__ void __launch_bounds__(BS)
+    k_face_flux(const __grid_constant__ OneRegion<R> regs, const Tile *__restrict__ tiles,
+                int nTiles, int pfDist) {
+  const int dist = (int)gridDim.x < nTiles ? (int)gridDim.x : pfDist;
+  RF_TILE_LOOP(pdl_wait(), nTiles) face_tile<R, BS, FPT>(regs, tiles, nTiles, t_, dist);
+}
+
+// FP64: one kernel for every launch shape, a tile of `stride` faces walked by
+// its block.  Bound by the FP64 pipe; 128 registers asked for (168: the same
+// time, 102: 1% slower).  64^3 tets AUSM+ 1.53 -> 1.11 ms, AUSM+up 1.76 ->
+// 1.32, Roe 2.42 -> 1.83, HLLC 1.82 -> 1.44 with the reconstruction and prod()
+// products on the integer pipes (the reconstruction alone: 1.32, 1.54, 2.14,
+// 1.60), the exponent scalings, and the velocities kept per cell.
+template <typename RT>
+__device__ __forceinline__ void face64_body(const RT &regs, const Tile *__restrict__ tiles,
+                                            int nTiles, int pfDist, int stride) {
+  const int dist = (int)gridDim.x < nTiles ? (int)gridDim.x : pfDist;
+  RF_TILE_LOOP(pdl_wait(), nTiles) {
+    const Tile tl = tile_at(regs, tiles, t_, stride);
+    const RegionDev<double> &g = regs[tl.region];
+    prefetch_ahead(t_, nTiles, dist, [&](int t) {
+      const Tile tp = tile_at(regs, tiles, t, stride);
+      prefetch_face_tile(regs[tp.region], tp.first, stride);
+    });
+    const int last = tl.first + stride < g.nFaces ? tl.first + stride : g.nFaces;
+    for (int f = tl.first + threadIdx.x; f < last; f += blockDim.x) face_flux_one(g, f);
+  }
+}
+template <typename R>
+__global__ void __launch_bounds__(128, 4)
+    k_face_flux64(const RegionDev<double> *__restrict__ regs, const Tile *__restrict__ tiles,
+                  int nTiles, int pfDist, int stride) {
+  face64_body(regs, tiles, nTiles, pfDist, stride);
+}
+template <typename R>
+__global__ void __launch_bounds__(128, 4)
+    k_face_flux64(const __grid_constant__ OneRegion<double> regs, const Tile *__restrict__ tiles,
+                  int nTiles, int pfDist, int stride) {
+  face64_body(regs, tiles, nTiles, pfDist, stride);
 }
 
 template <typename R>
@@ -2029,9 +2105,30 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 0 : 4))
       dt_finalize_block<R>(regs, x.nRegions, x.coupled, x.a, smin);
   }
 }
+template <typename R>
+__global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 0 : 4))
+    k_flux_merged(const __grid_constant__ OneRegion<R> regs, const Tile *__restrict__ tiles, int nTiles,
+                  int pfDist, const FluxExtra x) {
+  __shared__ unsigned long long smin[32];
+  const int n0 = x.dt + x.nBFace;
+  const int dist = (int)gridDim.x < nTiles + n0 ? (int)gridDim.x : pfDist;
+  RF_TILE_LOOP(pdl_wait(), nTiles + n0) {
+    if (t_ >= n0)
+      face_tile<R, 128, 1>(regs, tiles, nTiles, t_ - n0, dist);
+    else if (t_ >= x.dt)
+      bface_tile<R>(regs, x.bface, t_ - x.dt);
+    else
+      dt_finalize_block<R>(regs, x.nRegions, x.coupled, x.a, smin);
+  }
+}
 
 template <typename R>
 __global__ void __launch_bounds__(128) k_bface_flux(const RegionDev<R> *__restrict__ regs,
+                                                    const Tile *__restrict__ tiles, int nTiles) {
+  RF_TILE_LOOP(pdl_wait(), nTiles) bface_tile<R>(regs, tiles, t_);
+}
+template <typename R>
+__global__ void __launch_bounds__(128) k_bface_flux(const __grid_constant__ OneRegion<R> regs,
                                                     const Tile *__restrict__ tiles, int nTiles) {
   RF_TILE_LOOP(pdl_wait(), nTiles) bface_tile<R>(regs, tiles, t_);
 }
@@ -2480,15 +2577,14 @@ __device__ __forceinline__ void gather_update_split(const RegionDev<float> &g, i
 // residual is written (rfgpu_residual).
 // SPLIT selects the split path's update at compile time (a run-time branch
 // between the two FP32-flux updates costs the mixed path registers).
-template <typename R, int SPLIT>
-__device__ __forceinline__ void update_tile(const RegionDev<R> *__restrict__ regs,
-                                            const Tile *__restrict__ tiles, int nTiles, int t_,
-                                            const StepArgs &a, int dist) {
+template <typename R, int SPLIT, typename RT>
+__device__ __forceinline__ void update_tile(const RT &regs, const Tile *__restrict__ tiles,
+                                            int nTiles, int t_, const StepArgs &a, int dist) {
   {
-    const Tile tl = tiles[t_];
+    const Tile tl = tile_at(regs, tiles, t_, blockDim.x);
     const RegionDev<R> &g = regs[tl.region];
     prefetch_ahead(t_, nTiles, dist, [&](int t) {
-      const Tile tp = tiles[t];
+      const Tile tp = tile_at(regs, tiles, t, blockDim.x);
       prefetch_update_tile(regs[tp.region], tp.first);
     });
     const int c = tl.first + threadIdx.x;
@@ -2579,6 +2675,17 @@ template <typename R, int BS, int SPLIT>
 __global__ void __launch_bounds__(BS) k_gather_update(const RegionDev<R> *__restrict__ regs,
                                                       const Tile *__restrict__ tiles,
                                                       int nTiles, StepArgs a, int pfDist) {
+  const int dist = (int)gridDim.x < nTiles ? (int)gridDim.x : pfDist;
+  RF_TILE_LOOP(pdl_wait(), nTiles) update_tile<R, SPLIT>(regs, tiles, nTiles, t_, a, dist);
+}
+// One region, mixed: 10 blocks of 128 asked for (48 registers).  Update pass of
+// 12.6 M tets, 1.57 M tets and the 2.48 M-cell box: 0.591, 0.081, 0.100 ms; the
+// compiler's 64 registers 0.601, 0.086, 0.122; 9 blocks 0.599, 0.081, 0.106; 11
+// blocks 0.623, 0.084, 0.095; the table version 0.583, 0.084, 0.116.
+template <typename R, int BS, int SPLIT>
+__global__ void __launch_bounds__(BS, sizeof(R) == 4 && SPLIT == 0 ? 10 * 128 / BS : 0)
+    k_gather_update(const __grid_constant__ OneRegion<R> regs, const Tile *__restrict__ tiles,
+                    int nTiles, StepArgs a, int pfDist) {
   const int dist = (int)gridDim.x < nTiles ? (int)gridDim.x : pfDist;
   RF_TILE_LOOP(pdl_wait(), nTiles) update_tile<R, SPLIT>(regs, tiles, nTiles, t_, a, dist);
 }
@@ -2735,20 +2842,41 @@ void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, con
   cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
 }
 
+// The region argument of a launch: the descriptor where the Work is one region
+// (its own tile lists are then consecutive tiles), else the table.
+template <bool ONE = true, typename R, typename F>
+void with_regions(const RegionDev<R> *regs, const Work &w, const Tile *tiles, F f) {
+  if constexpr (ONE) {  // other launch shapes than the default keep the table
+    if (w.one) {
+      const bool own = tiles == w.cellTiles || tiles == w.faceTiles || tiles == w.bfaceTiles;
+      f(OneRegion<R>{*static_cast<const RegionDev<R> *>(w.one)}, own ? nullptr : tiles);
+      return;
+    }
+  }
+  f(regs, tiles);
+}
+
 template <typename R, int F, int BS>
-void grad_launch(const RegionDev<R> *regs, const Tile *tiles, int nTiles, int cap, cudaStream_t s) {
+void grad_launch(const RegionDev<R> *regs, const Work &w, const Tile *tiles, int nTiles, int cap,
+                 cudaStream_t s) {
   if constexpr (sizeof(R) == 8) {
     const int per = BS / 32, n = grid_for(cap, nTiles * per);
     if (n <= 0) return;
-    if (n == nTiles * per && n < kGrad64Rows)
-      launch_pdl(k_grad_lim64<F>, dim3(n, 5), dim3(32, 1), s, regs, tiles, nTiles, per);
-    else
-      launch_pdl(k_grad_lim64<F>, n, dim3(32, 5), s, regs, tiles, nTiles, per);
-    return;
+    const bool five = n == nTiles * per && n < kGrad64Rows;
+    with_regions(regs, w, tiles, [&](const auto &r, const Tile *t) {
+      using RA = std::decay_t<decltype(r)>;
+      launch_pdl(static_cast<void (*)(RA, const Tile *, int, int)>(k_grad_lim64<F>),
+                 dim3(n, five ? 5 : 1), dim3(32, five ? 1 : 5), s, r, t, nTiles, per);
+    });
+  } else {
+    const int grid = grid_for(cap, nTiles);
+    if (grid <= 0) return;
+    with_regions<BS == 128>(regs, w, tiles, [&](const auto &r, const Tile *t) {
+      using RA = std::decay_t<decltype(r)>;
+      launch_pdl(static_cast<void (*)(RA, const Tile *, int)>(k_grad_lim<R, F, BS>), grid, BS, s, r,
+                 t, nTiles);
+    });
   }
-  const int grid = grid_for(cap, nTiles);
-  if constexpr (sizeof(R) == 4)
-    if (grid > 0) launch_pdl(k_grad_lim<R, F, BS>, grid, BS, s, regs, tiles, nTiles);
 }
 
 template <typename R>
@@ -2758,22 +2886,43 @@ void launch_grad_tuned(const RegionDev<R> *regs, const Work &w, int fuseDt, cuda
   const int n = tuned ? w.nGradTiles : w.nCellTiles;
   const int bs = tuned ? w.gradBlock : 128;
   if (bs == 64) {
-    if (fuseDt) grad_launch<R, 1, 64>(regs, t, n, w.grid, s);
-    else grad_launch<R, 0, 64>(regs, t, n, w.grid, s);
+    if (fuseDt) grad_launch<R, 1, 64>(regs, w, t, n, w.grid, s);
+    else grad_launch<R, 0, 64>(regs, w, t, n, w.grid, s);
   } else if (bs == 256) {
-    if (fuseDt) grad_launch<R, 1, 256>(regs, t, n, w.grid, s);
-    else grad_launch<R, 0, 256>(regs, t, n, w.grid, s);
+    if (fuseDt) grad_launch<R, 1, 256>(regs, w, t, n, w.grid, s);
+    else grad_launch<R, 0, 256>(regs, w, t, n, w.grid, s);
   } else {
-    if (fuseDt) grad_launch<R, 1, 128>(regs, t, n, w.grid, s);
-    else grad_launch<R, 0, 128>(regs, t, n, w.grid, s);
+    if (fuseDt) grad_launch<R, 1, 128>(regs, w, t, n, w.grid, s);
+    else grad_launch<R, 0, 128>(regs, w, t, n, w.grid, s);
   }
 }
 
+template <typename R>
+void launch_face64(const RegionDev<R> *regs, const Work &w, const Tile *tiles, int nTiles, int grid,
+                   int block, int stride, cudaStream_t s) {
+  with_regions(regs, w, tiles, [&](const auto &r, const Tile *t) {
+    using RA = std::decay_t<decltype(r)>;
+    const auto k = static_cast<void (*)(RA, const Tile *, int, int, int)>(k_face_flux64<R>);
+    static const int pf = resident_blocks(k, 128);
+    launch_pdl(k, grid, block, s, r, t, nTiles, pf, stride);
+  });
+}
+
 template <typename R, int BS, int FPT>
-void face_launch(const RegionDev<R> *regs, const Tile *tiles, int nTiles, int cap, cudaStream_t s) {
-  static const int pf = resident_blocks(k_face_flux<R, BS, FPT>, BS);
-  const int grid = grid_for(cap, nTiles);
-  if (grid > 0) launch_pdl(k_face_flux<R, BS, FPT>, grid, BS, s, regs, tiles, nTiles, pf);
+void face_launch(const RegionDev<R> *regs, const Work &w, const Tile *tiles, int nTiles,
+                 cudaStream_t s) {
+  const int grid = grid_for(w.grid, nTiles);
+  if (grid <= 0) return;
+  if constexpr (sizeof(R) == 8) {
+    launch_face64<R>(regs, w, tiles, nTiles, grid, BS < 128 ? BS : 128, BS * FPT, s);
+  } else {
+    with_regions<BS == 128 && FPT == 1>(regs, w, tiles, [&](const auto &r, const Tile *t) {
+      using RA = std::decay_t<decltype(r)>;
+      const auto k = static_cast<void (*)(RA, const Tile *, int, int)>(k_face_flux<R, BS, FPT>);
+      static const int pf = resident_blocks(k, BS);
+      launch_pdl(k, grid, BS, s, r, t, nTiles, pf);
+    });
+  }
 }
 
 // The merged launch pays where the passes are short against their latency
@@ -2784,41 +2933,53 @@ void face_launch(const RegionDev<R> *regs, const Tile *tiles, int nTiles, int ca
 // the face pass more, 8.89 -> 8.93 ms.
 constexpr int kMergeTiles = 100000;
 template <typename R>
-void merged_launch(const RegionDev<R> *regs, const Work &w, const FluxExtra &x, cudaStream_t s) {
-  static const int pf = resident_blocks(k_flux_merged<R>, 128);
+void merged_launch(const RegionDev<R> *regs, const Work &w, FluxExtra x, cudaStream_t s) {
   const int grid = grid_for(w.grid, w.nFaceTiles + x.nBFace + x.dt);
-  launch_pdl(k_flux_merged<R>, grid, 128, s, regs, w.faceTiles, w.nFaceTiles, pf, x);
+  with_regions(regs, w, w.faceTiles, [&](const auto &r, const Tile *t) {
+    using RA = std::decay_t<decltype(r)>;
+    const auto k =
+        static_cast<void (*)(RA, const Tile *, int, int, const FluxExtra)>(k_flux_merged<R>);
+    static const int pf = resident_blocks(k, 128);
+    if (!t) x.bface = nullptr;  // consecutive tiles as well
+    launch_pdl(k, grid, 128, s, r, t, w.nFaceTiles, pf, x);
+  });
 }
 
 template <typename R>
 void launch_faces_tuned(const RegionDev<R> *regs, const Work &w, cudaStream_t s) {
   const int bs = w.faceBlock ? w.faceBlock : 128, fpt = w.facesPerThread ? w.facesPerThread : 1;
   if (bs == 64) {
-    if (fpt == 2) face_launch<R, 64, 2>(regs, w.faceTiles, w.nFaceTiles, w.grid, s);
-    else face_launch<R, 64, 1>(regs, w.faceTiles, w.nFaceTiles, w.grid, s);
+    if (fpt == 2) face_launch<R, 64, 2>(regs, w, w.faceTiles, w.nFaceTiles, s);
+    else face_launch<R, 64, 1>(regs, w, w.faceTiles, w.nFaceTiles, s);
   } else if (bs == 256) {
-    if (fpt == 2) face_launch<R, 256, 2>(regs, w.faceTiles, w.nFaceTiles, w.grid, s);
-    else face_launch<R, 256, 1>(regs, w.faceTiles, w.nFaceTiles, w.grid, s);
+    if (fpt == 2) face_launch<R, 256, 2>(regs, w, w.faceTiles, w.nFaceTiles, s);
+    else face_launch<R, 256, 1>(regs, w, w.faceTiles, w.nFaceTiles, s);
   } else {
-    if (fpt == 2) face_launch<R, 128, 2>(regs, w.faceTiles, w.nFaceTiles, w.grid, s);
-    else face_launch<R, 128, 1>(regs, w.faceTiles, w.nFaceTiles, w.grid, s);
+    if (fpt == 2) face_launch<R, 128, 2>(regs, w, w.faceTiles, w.nFaceTiles, s);
+    else face_launch<R, 128, 1>(regs, w, w.faceTiles, w.nFaceTiles, s);
   }
 }
 
 template <typename R, int BS, int SPLIT>
-void update_launch_k(const RegionDev<R> *regs, const Tile *tiles, int nTiles, int cap,
+void update_launch_k(const RegionDev<R> *regs, const Work &w, const Tile *tiles, int nTiles,
                      const StepArgs &a, cudaStream_t s) {
-  static const int pf = resident_blocks(k_gather_update<R, BS, SPLIT>, BS);
-  const int grid = grid_for(cap, nTiles);
-  if (grid > 0) launch_pdl(k_gather_update<R, BS, SPLIT>, grid, BS, s, regs, tiles, nTiles, a, pf);
+  const int grid = grid_for(w.grid, nTiles);
+  if (grid <= 0) return;
+  with_regions<BS == 128>(regs, w, tiles, [&](const auto &r, const Tile *t) {
+    using RA = std::decay_t<decltype(r)>;
+    const auto k =
+        static_cast<void (*)(RA, const Tile *, int, StepArgs, int)>(k_gather_update<R, BS, SPLIT>);
+    static const int pf = resident_blocks(k, BS);
+    launch_pdl(k, grid, BS, s, r, t, nTiles, a, pf);
+  });
 }
 template <typename R, int BS>
-void update_launch(const RegionDev<R> *regs, const Tile *tiles, int nTiles, int cap,
-                   const StepArgs &a, int split, cudaStream_t s) {
-  if (sizeof(R) == 4 && split)
-    update_launch_k<R, BS, 1>(regs, tiles, nTiles, cap, a, s);
-  else
-    update_launch_k<R, BS, 0>(regs, tiles, nTiles, cap, a, s);
+void update_launch(const RegionDev<R> *regs, const Work &w, const Tile *tiles, int nTiles,
+                   const StepArgs &a, cudaStream_t s) {
+  if constexpr (sizeof(R) == 4) {
+    if (w.split) return update_launch_k<R, BS, 1>(regs, w, tiles, nTiles, a, s);
+  }
+  update_launch_k<R, BS, 0>(regs, w, tiles, nTiles, a, s);
 }
 
 template <typename R>
@@ -2828,15 +2989,14 @@ void launch_update_tuned(const RegionDev<R> *regs, const Work &w, const StepArgs
   const Tile *t = tuned ? w.updTiles : w.cellTiles;
   const int n = tuned ? w.nUpdTiles : w.nCellTiles;
   const int bs = tuned ? w.cellBlock : 128;
-  if (bs == 64) update_launch<R, 64>(regs, t, n, w.grid, a, w.split, s);
-  else if (bs == 256) update_launch<R, 256>(regs, t, n, w.grid, a, w.split, s);
-  else update_launch<R, 128>(regs, t, n, w.grid, a, w.split, s);
+  if (bs == 64) update_launch<R, 64>(regs, w, t, n, a, s);
+  else if (bs == 256) update_launch<R, 256>(regs, w, t, n, a, s);
+  else update_launch<R, 128>(regs, w, t, n, a, s);
 }
 
 // ---- one launch per RK stage ---------------------------------------------------
-template <typename R>
-__device__ __forceinline__ void weno_tile(const RegionDev<R> *__restrict__ regs,
-                                          const Tile *__restrict__ tiles, int t_);
+template <typename R, typename RT>
+__device__ __forceinline__ void weno_tile(const RT &regs, const Tile *__restrict__ tiles, int t_);
 
 // Grid-wide barrier of the persistent stage kernel, a cooperative launch (so
 // every block is resident).  Thread 0 of each block arrives; the last arrival
@@ -2946,10 +3106,14 @@ void launch_stage(const RegionDev<R> *regs, const Work &w, const StepArgs &a, cu
     const int grad = spaceOrder > 1 && w.nCellTiles > 0;
     const int weno = grad && reconst == 2;
     RF_MARK(KP_STAGE, 0);
-    if (sizeof(R) == 4 && w.split)
-      coop_launch<R, 1>(regs, w, a, grad, weno, s);
-    else
+    if constexpr (sizeof(R) == 4) {
+      if (w.split)
+        coop_launch<R, 1>(regs, w, a, grad, weno, s);
+      else
+        coop_launch<R, 0>(regs, w, a, grad, weno, s);
+    } else {
       coop_launch<R, 0>(regs, w, a, grad, weno, s);
+    }
     RF_MARK(KP_STAGE, 1);
     if (launches) *launches += 1;
     return;
@@ -2995,7 +3159,7 @@ void launch_stage(const RegionDev<R> *regs, const Work &w, const StepArgs &a, cu
   }
   if (bface && !merge) {
     RF_MARK(KP_BFACE_FLUX, 0);
-    launch_pdl(k_bface_flux<R>, gsz(w.nBFaceTiles), w.block, s, regs, w.bfaceTiles, w.nBFaceTiles);
+    launch_bface_tiles<R>(regs, w, w.bfaceTiles, w.nBFaceTiles, s);
     RF_MARK(KP_BFACE_FLUX, 1);
     ++n;
   }
@@ -3055,11 +3219,10 @@ void launch_step(const RegionDev<R> *regs, const Work &w, const DtArgs &da, int 
 // var + grad . (fc - xc) is not positive at one of the cell's faces, interior
 // or boundary (the result does not depend on the face order).  Regions that
 // do not use RECONST 2 skip their tiles.
-template <typename R>
-__device__ __forceinline__ void weno_tile(const RegionDev<R> *__restrict__ regs,
-                                          const Tile *__restrict__ tiles, int t_) {
+template <typename R, typename RT>
+__device__ __forceinline__ void weno_tile(const RT &regs, const Tile *__restrict__ tiles, int t_) {
   {
-    const Tile tl = tiles[t_];
+    const Tile tl = tile_at(regs, tiles, t_, blockDim.x);
     const RegionDev<R> &g = regs[tl.region];
     if (!g.gradRaw) return;
     const int c = tl.first + threadIdx.x;
@@ -3207,9 +3370,20 @@ __global__ void __launch_bounds__(128) k_weno_xyz(const RegionDev<R> *__restrict
                                                   const Tile *__restrict__ tiles, int nTiles) {
   RF_TILE_LOOP(pdl_wait(), nTiles) weno_tile<R>(regs, tiles, t_);
 }
+template <typename R>
+__global__ void __launch_bounds__(128) k_weno_xyz(const __grid_constant__ OneRegion<R> regs,
+                                                  const Tile *__restrict__ tiles, int nTiles) {
+  RF_TILE_LOOP(pdl_wait(), nTiles) weno_tile<R>(regs, tiles, t_);
+}
 template <int MINB>
 __global__ void __launch_bounds__(128, MINB)
     k_weno_xyz_f32(const RegionDev<float> *__restrict__ regs, const Tile *__restrict__ tiles,
+                   int nTiles) {
+  RF_TILE_LOOP(pdl_wait(), nTiles) weno_tile<float>(regs, tiles, t_);
+}
+template <int MINB>
+__global__ void __launch_bounds__(128, MINB)
+    k_weno_xyz_f32(const __grid_constant__ OneRegion<float> regs, const Tile *__restrict__ tiles,
                    int nTiles) {
   RF_TILE_LOOP(pdl_wait(), nTiles) weno_tile<float>(regs, tiles, t_);
 }
@@ -3218,10 +3392,13 @@ template <typename R>
 void launch_weno_xyz(const RegionDev<R> *regs, const Work &w, cudaStream_t s) {
   if (w.nCellTiles <= 0) return;
   const int grid = w.grid > 0 && w.grid < w.nCellTiles ? w.grid : w.nCellTiles;
-  if constexpr (sizeof(R) == 4)
-    launch_pdl(k_weno_xyz_f32<RF_WENO_MINB>, grid, w.block, s, regs, w.cellTiles, w.nCellTiles);
-  else
-    launch_pdl(k_weno_xyz<R>, grid, w.block, s, regs, w.cellTiles, w.nCellTiles);
+  with_regions(regs, w, w.cellTiles, [&](const auto &r, const Tile *t) {
+    using K = void (*)(std::decay_t<decltype(r)>, const Tile *, int);
+    if constexpr (sizeof(R) == 4)
+      launch_pdl(static_cast<K>(k_weno_xyz_f32<RF_WENO_MINB>), grid, w.block, s, r, t, w.nCellTiles);
+    else
+      launch_pdl(static_cast<K>(k_weno_xyz<R>), grid, w.block, s, r, t, w.nCellTiles);
+  });
 }
 
 template <typename R>
@@ -3229,22 +3406,22 @@ void launch_grad_tiles(const RegionDev<R> *regs, const Work &w, const Tile *tile
                        int fuseDt, cudaStream_t s) {
   // the phase tile lists hold 128-cell tiles
   if (fuseDt)
-    grad_launch<R, 1, 128>(regs, tiles, nTiles, w.grid, s);
+    grad_launch<R, 1, 128>(regs, w, tiles, nTiles, w.grid, s);
   else
-    grad_launch<R, 0, 128>(regs, tiles, nTiles, w.grid, s);
+    grad_launch<R, 0, 128>(regs, w, tiles, nTiles, w.grid, s);
 }
 
 template <typename R>
 void launch_face_tiles(const RegionDev<R> *regs, const Work &w, const Tile *tiles, int nTiles,
                        cudaStream_t s) {
   // the phase lists hold 128-face tiles, one face per thread
-  if (nTiles > 0) face_launch<R, 128, 1>(regs, tiles, nTiles, w.grid, s);
+  if (nTiles > 0) face_launch<R, 128, 1>(regs, w, tiles, nTiles, s);
 }
 
 template <typename R>
 void launch_update_tiles(const RegionDev<R> *regs, const Work &w, const Tile *tiles, int nTiles,
                          const StepArgs &a, cudaStream_t s) {
-  update_launch<R, 128>(regs, tiles, nTiles, w.grid, a, w.split, s);  // 128-cell phase tiles
+  update_launch<R, 128>(regs, w, tiles, nTiles, a, s);  // 128-cell phase tiles
 }
 
 // The transfer chunk a host cell travels in.
@@ -3327,7 +3504,12 @@ template <typename R>
 void launch_bface_tiles(const RegionDev<R> *regs, const Work &w, const Tile *tiles, int nTiles,
                         cudaStream_t s) {
   const int grid = grid_for(w.grid, nTiles);
-  if (grid > 0) launch_pdl(k_bface_flux<R>, grid, w.block, s, regs, tiles, nTiles);
+  if (grid <= 0) return;
+  with_regions(regs, w, tiles, [&](const auto &r, const Tile *t) {
+    using RA = std::decay_t<decltype(r)>;
+    launch_pdl(static_cast<void (*)(RA, const Tile *, int)>(k_bface_flux<R>), grid, w.block, s, r, t,
+               nTiles);
+  });
 }
 
 template <typename R>
@@ -3425,12 +3607,12 @@ template <typename R>
 void launch_residual_scratch(const RegionDev<R> *regs, const RegionDev<R> &g, const Work &w,
                              int spaceOrder, R *flux, double *rhs, cudaStream_t s) {
   if (spaceOrder > 1 && w.nCellTiles > 0) {
-    grad_launch<R, 0, 128>(regs, w.cellTiles, w.nCellTiles, 0, s);
+    grad_launch<R, 0, 128>(regs, w, w.cellTiles, w.nCellTiles, 0, s);
     if (g.gradRaw) launch_weno_xyz<R>(regs, w, s);
   }
   if (g.nFaces > 0) k_face_flux_scratch<R><<<(g.nFaces + 127) / 128, 128, 0, s>>>(g, flux);
   if (w.nBFaceTiles > 0)
-    launch_pdl(k_bface_flux<R>, w.nBFaceTiles, w.block, s, regs, w.bfaceTiles, w.nBFaceTiles);
+    launch_bface_tiles<R>(regs, w, w.bfaceTiles, w.nBFaceTiles, s);
   k_gather_rhs_scratch<R><<<(g.nCells + 127) / 128, 128, 0, s>>>(g, flux, rhs);
 }
 
