@@ -1518,6 +1518,21 @@ __global__ void __launch_bounds__(160, 6)
   grad64_body<FUSE_DT>(regs, tiles, nTiles, per);
 }
 
+// Small single regions, mixed path: latency bounds the pass, not the number of
+// resident warps, so it takes 128 registers, which hold the eight gathers of a
+// group in flight (64 serialise them), and blocks of 64 cells, which spread over
+// the SMs.  A step of 3,000 / 10,000 / 25,000 / 48,000 tets: 61.4 / 61.5 / 65.6
+// / 73.7 -> 54.7 / 55.3 / 59.4 / 71.0 us; at 105,000 tets the resident warps
+// count again (108 -> 127 us).  Blocks of 32 and 128 measured the same within
+// 2%, 20 gathers in flight slower.
+constexpr int kFewBlock = 64, kFewTiles = 400;  // 128-cell tiles
+template <typename R, int FUSE_DT>
+__global__ void __launch_bounds__(kFewBlock, 8)
+    k_grad_few(const __grid_constant__ OneRegion<R> regs, int nTiles) {
+  __shared__ unsigned long long smin[32];
+  RF_TILE_LOOP(pdl_wait(), nTiles) grad_tile<R, FUSE_DT>(regs, nullptr, t_, smin);
+}
+
 template <typename R, int FUSE_DT, int BS>
 __global__ void __launch_bounds__(BS, ((sizeof(R) == 4) ? (FUSE_DT ? RF_GRAD_MINB_DT : RF_GRAD_MINB)
                                                         : 4) * 128 / BS)
@@ -2881,6 +2896,14 @@ void grad_launch(const RegionDev<R> *regs, const Work &w, const Tile *tiles, int
   } else {
     const int grid = grid_for(cap, nTiles);
     if (grid <= 0) return;
+    if constexpr (BS == 128) {
+      if (w.one && tiles == w.cellTiles && cap == 0 && nTiles < kFewTiles) {
+        const RegionDev<R> &d = *static_cast<const RegionDev<R> *>(w.one);
+        const int n = (d.nCells + kFewBlock - 1) / kFewBlock;
+        launch_pdl(k_grad_few<R, F>, n, kFewBlock, s, OneRegion<R>{d}, n);
+        return;
+      }
+    }
     with_regions<BS == 128>(regs, w, tiles, [&](const auto &r, const Tile *t) {
       using RA = std::decay_t<decltype(r)>;
       launch_pdl(static_cast<void (*)(RA, const Tile *, int)>(k_grad_lim<R, F, BS>), grid, BS, s, r,
