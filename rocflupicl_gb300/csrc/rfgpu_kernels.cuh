@@ -1917,16 +1917,16 @@ __device__ __forceinline__ void bcond_outflow(int bcOpt, R pout, R sxn, R syn, R
 // rocflu/RFLU_CentralFirstPatch.F90:575-946 (ORDER 1).  Slip walls store -0.0
 // as mass flux, the exact additive identity, since the reference leaves the
 // mass residual untouched there.
-constexpr int kBTile = 128;  // boundary faces per tile, whatever the block size
+constexpr int kBTile = 128;  // boundary faces per tile and threads of the blocks that take it
 template <typename R, typename RT>
 __device__ __forceinline__ void bface_tile(const RT &regs, const Tile *__restrict__ tiles, int t_) {
   {
     const Tile tl = tile_at(regs, tiles, t_, kBTile);
     const RegionDev<R> &g = regs[tl.region];
+    const int b = tl.first + threadIdx.x;
     const int B = g.nBFaces;
-    const int last = tl.first + kBTile < B ? tl.first + kBTile : B;
+    if (b >= B) return;
     const int N = g.nCells;
-    for (int b = tl.first + threadIdx.x; b < last; b += blockDim.x) {
     const int c = g.bf2c[b];
     const int kind = g.bkind[b];
     const int type = kind & 15, order = (kind >> 4) & 15, opt = kind >> 8;
@@ -2049,7 +2049,6 @@ __device__ __forceinline__ void bface_tile(const RT &regs, const Tile *__restric
     }
     flx[5] = flx[6] = flx[7] = R(0);
     st8(g.bflux + 8 * (size_t)b, flx);
-    }
   }
 }
 
