@@ -258,9 +258,11 @@ typedef struct {
                           the tile count walks the tiles persistently; 0 = one
                           block per tile */
   int gradBlock;       /* threads (= cells) per block of the gradient + limiter
-                          pass: 64, 128 (default) or 256 */
+                          pass: 64, 128 (default) or 256 (the FP64 path runs a
+                          warp per 32 cells and variable whatever it is) */
   int faceBlock;       /* threads per block of the interior-face flux pass: 64,
-                          128 (default) or 256 */
+                          128 (default) or 256 (FP64 path: 128 at most, walking
+                          the same tile) */
   int facesPerThread;  /* interior faces per thread of that pass: 1 (default) or 2 */
   int cellBlock;       /* threads (= cells) per block of the residual gather and
                           update pass: 64, 128 (default) or 256 */
