@@ -1115,7 +1115,8 @@ __device__ __forceinline__ float narrow_bits(double x, bool &ok) {
 // Screening of one variable's Venkatakrishnan terms.  In FP32 a term's
 // numerator and denominator are sums of terms of one sign (d2 and its bound dm
 // have the same sign), so its relative error stays below 3e-6 when nothing
-// leaves FP32's normal range; two terms further apart than 1e-5 are then
+// leaves FP32's normal range, the quotient included (at an extremum, dm = 0, it
+// is epsq / 2 d2^2); two terms further apart than 1e-5 are then
 // ordered as in FP64, and only the smallest one decides the limiter.  What the
 // screen cannot order - two different d2 within 1e-5, magnitudes outside the
 // ranges below, the reference's cancelling guard - is left to the FP64 loop.
@@ -1134,6 +1135,7 @@ __device__ __forceinline__ void venkat_screen(VenkatScreen &s, double d2, float 
   const float den0 = x * (fmaf(2.f * x, x, a) + xm), mag = fabsf(den0);
   ok = ok && mag > 1e-30f && mag < 1e30f && (pos || guard || mag > 1e-6f);
   const float t = __fdividef(num, den0 + ((pos || !guard) ? 1e-12f : -1e-12f));
+  ok = ok && t > 1e-36f;
   if (__double_as_longlong(d2) != __double_as_longlong(s.d2)) {  // an equal d2 has an equal term
     s.second = fminf(s.second, fmaxf(s.best, t));
     if (t < s.best) {
