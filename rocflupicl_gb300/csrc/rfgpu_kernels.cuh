@@ -2199,6 +2199,16 @@ __device__ __forceinline__ unsigned after_update(double gc, double gg, double q[
   return st;
 }
 
+// Whether after_update can change a cell or set a bit, apart from NaN
+// velocities and temperatures: not when density, pressure and energy are
+// positive and the pressure is no cancellation residue.  after_update forms the
+// pressure again in another order of operations, and only beyond 2^-30 of the
+// total energy are both sure to be positive.
+__device__ __forceinline__ bool checks_can_act(const double q[5], double p) {
+  return !positive_bits(q[0]) || !positive_bits(p) || !positive_bits(q[4]) ||
+         (unsigned)__double2hiint(p) + (30u << 20) < (unsigned)__double2hiint(q[4]);
+}
+
 // Error-free transformation of a + b (Knuth's TwoSum); lo collects the
 // rounding errors, so hi + lo carries about twice the FP32 significand.
 __device__ __forceinline__ void two_sum_acc(float &hi, float &lo, float x) {
@@ -2505,8 +2515,8 @@ __device__ __forceinline__ void eos_cell64(const Phys &ph, const double q[5], do
 // reference's operation order except that a*dt/V is a*dt times the stored
 // 1/V.  The FP32 record (rho, u, v, w, p) for the next stage's gathers is
 // rounded from the FP64 values.  AfterUpdateMP's checks
-// (libfloflu/AfterUpdateMP.F90:134-136) change nothing and set no bit when
-// rho > 0, p > 0 and the velocities are not NaN, so only other cells run them.
+// (libfloflu/AfterUpdateMP.F90:134-136) run only on cells they can act on
+// (checks_can_act; finite momenta over a normal density give no NaN).
 __device__ __forceinline__ void gather_update_split(const RegionDev<float> &g, int c,
                                                     const StepArgs &a) {
   const int N = g.nCells;
@@ -2579,8 +2589,7 @@ __device__ __forceinline__ void gather_update_split(const RegionDev<float> &g, i
   }
   double ir;
   double p = eos_p(ph, q, ir);
-  if (!positive_bits(q[0]) || !positive_bits(p) || !finite_bits(q[1]) || !finite_bits(q[2]) ||
-      !finite_bits(q[3])) {
+  if (checks_can_act(q, p) || !finite_bits(q[1]) || !finite_bits(q[2]) || !finite_bits(q[3])) {
     double d[3];
     d[0] = p;
     d[1] = p / (q[0] * ph.gvR);
@@ -2674,13 +2683,8 @@ __device__ __forceinline__ void update_tile(const RT &regs, const Tile *__restri
     eos_cell64(ph, q, ir, d[0], vel);
     d[1] = d[0] / (q[0] * gc);
     d[2] = sqrt(gg * gc * d[1]);
-    // AfterUpdateMP's checks change nothing and set no bit when density and
-    // pressure are positive, nothing is NaN and the pressure is no cancellation
-    // residue (it is recomputed there in another order: beyond 2^-30 of the
-    // total energy both are positive), so only other cells run them
-    if (!positive_bits(q[0]) || !positive_bits(d[0]) || !positive_bits(q[4]) ||
-        (unsigned)__double2hiint(d[0]) + (30u << 20) < (unsigned)__double2hiint(q[4]) ||
-        nan_bits(d[1]) || nan_bits(vel[0]) || nan_bits(vel[1]) || nan_bits(vel[2])) {
+    if (checks_can_act(q, d[0]) || nan_bits(d[1]) || nan_bits(vel[0]) || nan_bits(vel[1]) ||
+        nan_bits(vel[2])) {
       const unsigned st = after_update(gc, gg, q, d);
       if (st) atomicOr(g.status, st);
     }
