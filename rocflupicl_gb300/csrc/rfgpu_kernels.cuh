@@ -2968,13 +2968,11 @@ void face_launch(const RegionDev<R> *regs, const Work &w, const Tile *tiles, int
   }
 }
 
-// The merged launch pays where the passes are short against their latency
-// (ms per step, separate -> merged: 512 cells 0.0457 -> 0.0353 a residual,
-// 4,000-cell tube FP64 0.166 -> 0.131, 10,000 tets 0.082 -> 0.071, 197,000
-// tets 0.330 -> 0.313, 1.57 M tets WENO 2.340 -> 2.325, 3.07 M tets 2.349 ->
-// 2.345); on 12.6 M tets (196,000 tiles) the boundary code's registers cost
-// the face pass more, 8.89 -> 8.93 ms.
-constexpr int kMergeTiles = 100000;
+// The merged launch is never the slower one beyond 0.1% (ms per step, separate
+// -> merged: 512 cells 0.0457 -> 0.0353 a residual, 4,000-cell tube FP64 0.166
+// -> 0.131, 10,000 tets 0.082 -> 0.071, 197,000 tets 0.330 -> 0.313, 6.75 M tets
+// 4.571 -> 4.547, split 6.130 -> 6.075, 12.6 M tets 8.099 -> 8.072, split
+// 11.04 -> 10.95; FP64 8.4 M tets 81.52 -> 81.59).
 template <typename R>
 void merged_launch(const RegionDev<R> *regs, const Work &w, FluxExtra x, cudaStream_t s) {
   const int grid = grid_for(w.grid, w.nFaceTiles + x.nBFace + x.dt);
@@ -3206,7 +3204,7 @@ void launch_stage(const RegionDev<R> *regs, const Work &w, const StepArgs &a, cu
   const bool dt = a.fuseDt && hasGrad && flux, bface = flux && w.nBFaceTiles > 0;
   const bool faces = flux && !(parts & SP_NOFACE) && w.nFaceTiles > 0;
   const bool tuned = w.faceBlock != 0 && (w.faceBlock != 128 || w.facesPerThread != 1);
-  const bool merge = faces && !prof && !tuned && (dt || bface) && w.nFaceTiles < kMergeTiles;
+  const bool merge = faces && !prof && !tuned && (dt || bface);
   if (dt && !merge) {
     RF_MARK(KP_DT_FINAL, 0);
     launch_dt_finalize<R>(regs, w, a.dt, s);
