@@ -246,7 +246,15 @@ long long rfgpu_device_bytes(rfgpu_region_t h);
 /* Kernel launches issued by the handle since creation. */
 long long rfgpu_launch_count(rfgpu_region_t h);
 /* Launch shapes of the stage passes, chosen by the autotuner
- * (rocflupicl_gb300/autotune.py) by timing real steps.  Block sizes, faces per
+ * (rocflupicl_gb300/autotune.py) by timing real steps.  The default shapes
+ * have launches that others give up: a gradBlock, faceBlock, facesPerThread or
+ * cellBlock other than the default makes its pass read the region's descriptor
+ * from memory instead of its launch parameters (on the FP64 path cellBlock's
+ * alone), a
+ * faceBlock or facesPerThread other than the default also launches interior
+ * faces, boundary faces and the time step's finalisation one by one, and a
+ * gradBlock or gridCap other than the default forgoes the gradient pass for
+ * regions of at most 51,072 cells (reduced-precision paths).  Block sizes, faces per
  * thread and the grid leave every result bit for bit unchanged; the persistent
  * stage does on the FP64 path, and on the reduced-precision paths changes
  * results by FP32 rounding at most (the compiler may contract a product into
@@ -280,7 +288,9 @@ int rfgpu_set_tuning(rfgpu_region_t h, const rfgpu_tuning_t *t);
 
 /* Per-kernel profiler (the engine's counterpart of the reference's ROCPROF
  * FPROFILER_BEGINS/ENDS markers): while enabled, CUDA events are recorded on
- * the handle's stream around every kernel; rfgpu_profile_read synchronises and
+ * the handle's stream around every kernel, and the flux passes of a stage,
+ * otherwise one launch, are launched one by one: the times are the passes'
+ * own, their sum more than an unprofiled step; rfgpu_profile_read synchronises and
  * returns, per kernel class, the summed milliseconds and launch counts, then
  * resets.  Classes: 0 gradient, 1 limiter, 2 face flux, 3 boundary-face flux,
  * 4 gather+update, 5 dt faces, 6 dt boundary faces, 7 dt cells, 8 dt finalize,

@@ -18,8 +18,12 @@ by timing real steps on the device:
 The search is coordinate descent from the default shape: each knob in turn
 takes its candidates with the others fixed, judged by the CUDA-event time of
 the pass it shapes (the engine's per-kernel profiler, on the handle's stream)
-or, for the grid, of the whole step; the best is kept.  The steps taken while
-tuning advance the solution like any other step.
+or, for the grid, of the whole step; the best is kept.  While the profiler is
+on every pass is a launch of its own, and shapes other than the default give
+up launches that only the default has (include/rfgpu.h), so pass times only
+order the candidates: whole steps are timed without the profiler, and the
+shape found is kept only if its step is faster than the default shape's.  The
+steps taken while tuning advance the solution like any other step.
 """
 from __future__ import annotations
 
@@ -42,17 +46,37 @@ def _measure(h, shape: Dict[str, int], step, steps: int, kernel) -> float:
     h.set_tuning(**shape)
     step()                                  # settle (first launch of a shape)
     h.sync()
-    h.profile(True)
+    if kernel is not None:
+        h.profile(True)
     h.timer_start()
     for _ in range(steps):
         step()
     ms = h.timer_stop()
-    prof = h.profile_read()
-    h.profile(False)
     if kernel is None:
         return ms / steps
+    prof = h.profile_read()
+    h.profile(False)
     t, n = prof.get(kernel, (0.0, 0))
     return t / max(n, 1) if n else ms / steps
+
+
+def _or_default(h, out: Dict[str, object], step, steps: int,
+                grid_cap: int = 0) -> Dict[str, object]:
+    """The shape of a descent if its whole step is faster than that of the
+    default shape (with the grid cap given), else the default; both timed in
+    turn, twice."""
+    shape, default = out["shape"], dict({k: 0 for k in E.TUNING_KEYS}, gridCap=grid_cap)
+    n = max(steps, 5)
+    ms = {"default": float("inf"), "tuned": float("inf")}
+    for _ in range(2):
+        for name, s in (("default", default), ("tuned", shape)):
+            ms[name] = min(ms[name], _measure(h, s, step, n, None))
+            out["steps_taken"] += n + 1
+    out["ms"]["shape"] = ms
+    if not ms["tuned"] < ms["default"]:
+        out["shape"] = default
+    h.set_tuning(**out["shape"])
+    return out
 
 
 def _descend(h, step, steps: int, knobs: Dict[str, Sequence[int]],
@@ -95,8 +119,8 @@ def tune_region(region: "E.Region", cfl: float, dt_imposed: float, end_time: flo
         grid_caps = [0] + [sms * k for k in (4, 8, 16)]
     knobs = {"gradBlock": BLOCKS, "faceBlock": BLOCKS, "facesPerThread": (1, 2),
              "cellBlock": BLOCKS, "gridCap": grid_caps}
-    out = _descend(region, lambda: region.step(cfl, dt_imposed, 0.0, end_time), steps, knobs,
-                   persistent=True)
+    step = lambda: region.step(cfl, dt_imposed, 0.0, end_time)  # noqa: E731
+    out = _or_default(region, _descend(region, step, steps, knobs, persistent=True), step, steps)
     out["sms"] = sms
     return out
 
@@ -113,8 +137,11 @@ def tune_batch(batch: "E.Batch", cfl: float, dt_imposed: float = 1.0, end_time: 
     if blocks:
         knobs.update({"gradBlock": BLOCKS, "faceBlock": BLOCKS, "facesPerThread": (1, 2),
                       "cellBlock": BLOCKS})
-    out = _descend(batch, lambda: batch.step(cfl, dt_imposed, 0.0, end_time), steps, knobs,
-                   persistent=True)
+    step = lambda: batch.step(cfl, dt_imposed, 0.0, end_time)  # noqa: E731
+    out = _descend(batch, step, steps, knobs, persistent=True)
+    # the grid caps were timed on the default blocks, the engine's own among them
+    caps = out["ms"]["gridCap"]
+    out = _or_default(batch, out, step, steps, grid_cap=min(caps, key=caps.get))
     out["sms"] = sms
     out["grid_cap"] = out["shape"]["gridCap"]
     out["ms_per_step"] = out["ms"]["gridCap"]
