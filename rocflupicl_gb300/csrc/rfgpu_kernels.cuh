@@ -512,18 +512,18 @@ __device__ __forceinline__ void reconstruct(const R G[16], R dx, R dy, R dz, R S
 // One face term of RFLU_ComputeLimiterVenkat (modflu/RFLU_ModLimiters.F90:482-504).
 // guard = 0 keeps the reference's denom + TINY; guard = 1 adds TINY with the
 // sign of denom (for d2 < 0 the reference sum can cancel).
-// Mixed path: the quotient is the hardware approximate division
-// (__fdividef, within 2 ulp for denominators below 2^126; the terms here stay
-// far below), measured on the 128^3 tet box: gradient pass 1.838 -> 1.814 ms;
-// the FP64 path keeps IEEE division.
+// Mixed path: the quotient is a times the hardware reciprocal of b, within
+// 2^-23 + 2^-24 (12.6 M tets, gradient pass: IEEE division 1.838 ms, __fdividef
+// 1.814; on the later kernel __fdividef 1.570, this 1.561); the FP64 path keeps
+// IEEE division.
 #ifndef RF_LIM_FASTDIV
 #define RF_LIM_FASTDIV 1
 #endif
-// The hardware reciprocal.  __fdividef(a, b) is a times it with a rescaling for
-// |b| > 2^126, where both give 0 all the same, and for subnormal b, which the
-// denominators here never are: the same bits with fewer instructions (12.6 M
-// tets, gradient pass 1.570 -> 1.561 ms; WENO pass of 1.57 M tets 0.396 ->
-// 0.383).
+// The hardware reciprocal: by the PTX manual a relative error of at most 2^-23,
+// subnormal operands and results taken as zero.  The limiter's denominators are
+// sums with a 1e-12, zero or normal; beyond 2^126 the reciprocal and the term
+// are zero, as the programming guide has them for __fdividef.  WENO pass of 1.57
+// M tets: __fdividef 0.396 ms, this 0.383.
 __device__ __forceinline__ float rcp_ftz(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
