@@ -822,19 +822,19 @@ const RegionDev<R> *regs_of(rfgpu_region_s *h) {
   return (const RegionDev<R> *)h->regsDev;
 }
 
-constexpr int kXChunks = 8;  // transfer chunks of the mixed path
+constexpr int kXChunks = 8;  // transfer chunks of the mixed path, at most
 
 // Tiles [t0, t1) of chunk k, and its host cells [c0, c1).  With the full 8
 // chunks the first and last are smaller (weights 1,2,3,3,3,3,2,1): the first
 // download copy starts sooner and the work left after the last upload copy is
 // shorter (measured on 12.6 M cells: rfgpu_step_host 14.19 -> 14.11 ms, upload
-// + step + download 16.19 -> 16.08 ms against even chunks); regions under 36
-// tiles get even chunks.
+// + step + download 16.19 -> 16.08 ms against even chunks); fewer chunks are
+// even.
 void chunk_range(const rfgpu_region_s *h, int k, int nk, int &t0, int &t1, size_t &c0,
                  size_t &c1) {
   const int nT = h->work.nCellTiles;
   static const int cum[kXChunks + 1] = {0, 1, 3, 6, 9, 12, 15, 17, 18};
-  if (nk == kXChunks && nT >= 2 * cum[kXChunks]) {
+  if (nk == kXChunks) {
     t0 = (int)((long long)nT * cum[k] / cum[kXChunks]);
     t1 = (int)((long long)nT * cum[k + 1] / cum[kXChunks]);
   } else {
@@ -846,7 +846,8 @@ void chunk_range(const rfgpu_region_s *h, int k, int nk, int &t0, int &t1, size_
 }
 
 // Chunks of a transfer.  A chunk costs a copy, two events and a launch or two
-// whatever its size, so one holds 131,072 cells or more.  Against 8 chunks for
+// whatever its size, so they hold 131,072 cells or more on average, and two
+// million cells or more make the full 8.  Against 8 chunks for
 // every region: host-resident step of 10,000 cells 295 -> 112 us, 48,000 349 ->
 // 146, 280,000 604 -> 459; upload of 10,000 cells 54 -> 20 us.  6 chunks for
 // 1.57 M cells: 1.72 ms against 1.78 with 8; the same at 3.07 M.

@@ -695,7 +695,7 @@ __device__ __forceinline__ Tile tile_at(const OneRegion<R> &, const Tile *__rest
 
 // Cons2Prim (modflu/RFLU_ModConvertCv.F90:221-231) of one cell's FP64 state
 // into its record, and optionally the EOS first (libflu/RFLU_SetDependentVars.F90:
-// 256-287).  The record's centroid slots are kept.  FP64 path.
+// 256-287).  FP64 path: every slot of the record is written (trip_velocity).
 template <typename R>
 __device__ __forceinline__ void set_vars_cell(const RegionDev<R> &g, int c, int computeDv) {
   const int N = g.nCells;
@@ -713,7 +713,7 @@ __device__ __forceinline__ void set_vars_cell(const RegionDev<R> &g, int c, int 
     g.dv[2 * N + c] = sqrt(gg * gc * T);
   }
   R r[8];
-  ld8_rw(g.rec + 8 * (size_t)c, r);
+  if constexpr (sizeof(R) == 4) ld8_rw(g.rec + 8 * (size_t)c, r);
   r[0] = R(q0);
   r[1] = R(ir * q1);
   r[2] = R(ir * q2);
@@ -1090,7 +1090,7 @@ __device__ __forceinline__ double cell_dt(const RegionDev<R> &g, int c, const R 
 // the same bits), the min / max comparisons run on the bit patterns, and the
 // limiter's quotients are first formed in FP32 to find the face that decides
 // each variable's minimum, whose quotient alone is then formed in FP64.
-// FP64 operations per tet cell with 40 members: about 980 against 2440.
+// FP64 operations per tet cell with 40 members: about 975 against 2440.
 
 // b < a for numbers that are neither infinite nor NaN.  (-0 counts as below
 // +0; a zero's sign never reaches the limiter's result.)
@@ -1468,7 +1468,7 @@ __device__ __forceinline__ void grad_tile(const RT &regs, const Tile *__restrict
 }
 
 // FP64: one warp per 32 cells and variable, so that a region of a few thousand
-// cells reaches every SM quarter's FP64 unit and a large one needs 80 registers
+// cells reaches every SM quarter's FP64 unit and a large one needs 64 registers
 // a thread instead of 128.  Measured (pass with its launch): 512 cells 48.8 ->
 // 22.8 us, 4,000 cells 49.0 -> 22.9, 64,000 cells 98 -> 66, 1.57 M cells 6.08
 // -> 3.24 ms, about 975 FP64 operations per cell at 0.51 T/s (one thread per
@@ -1596,10 +1596,6 @@ __device__ __forceinline__ void face_riemann(const RegionDev<R> &g, int c1, int 
   }
 }
 
-// Interior face fluxes, *_ComputeFlux2_TCP face loops (AUSM+ :2726-2846,
-// Roe :2646-2855, HLLC :2239-2409), written to the face flux buffer.  A tile
-// is BS * FPT consecutive faces; thread i of the block takes faces i, i + BS,
-// ... of it (FPT faces per thread).
 // Flux of one interior face in the arithmetic type A (R, or Sd for R = double).
 template <typename A, typename R>
 __device__ __forceinline__ void face_flux_in(const RegionDev<R> &g, int f, int c1, int c2,
@@ -1673,6 +1669,10 @@ __device__ __forceinline__ void face_flux_one(const RegionDev<R> &g, int f) {
   }
 }
 
+// Interior face fluxes, *_ComputeFlux2_TCP face loops (AUSM+ :2726-2846,
+// Roe :2646-2855, HLLC :2239-2409), written to the face flux buffer.  A tile
+// is BS * FPT consecutive faces; thread i of the block takes faces i, i + BS,
+// ... of it (FPT faces per thread).
 template <typename R, int BS, int FPT, typename RT>
 __device__ __forceinline__ void face_tile(const RT &regs, const Tile *__restrict__ tiles,
                                           int nTiles, int t_, int dist) {
@@ -2114,11 +2114,10 @@ __global__ void __launch_bounds__(128, 4)
   face64_body(regs, tiles, nTiles, pfDist, stride);
 }
 
-template <typename R>
-__global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 0 : 4))
-    k_flux_merged(const RegionDev<R> *__restrict__ regs, const Tile *__restrict__ tiles, int nTiles,
-                  int pfDist, const FluxExtra x) {
-  __shared__ unsigned long long smin[32];
+template <typename R, typename RT>
+__device__ __forceinline__ void flux_merged_body(const RT &regs, const Tile *__restrict__ tiles,
+                                                 int nTiles, int pfDist, const FluxExtra &x,
+                                                 unsigned long long *smin) {
   const int n0 = x.dt + x.nBFace;
   const int dist = (int)gridDim.x < nTiles + n0 ? (int)gridDim.x : pfDist;
   RF_TILE_LOOP(pdl_wait(), nTiles + n0) {
@@ -2132,19 +2131,17 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 0 : 4))
 }
 template <typename R>
 __global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 0 : 4))
+    k_flux_merged(const RegionDev<R> *__restrict__ regs, const Tile *__restrict__ tiles, int nTiles,
+                  int pfDist, const FluxExtra x) {
+  __shared__ unsigned long long smin[32];
+  flux_merged_body<R>(regs, tiles, nTiles, pfDist, x, smin);
+}
+template <typename R>
+__global__ void __launch_bounds__(128, (sizeof(R) == 4 ? 0 : 4))
     k_flux_merged(const __grid_constant__ OneRegion<R> regs, const Tile *__restrict__ tiles, int nTiles,
                   int pfDist, const FluxExtra x) {
   __shared__ unsigned long long smin[32];
-  const int n0 = x.dt + x.nBFace;
-  const int dist = (int)gridDim.x < nTiles + n0 ? (int)gridDim.x : pfDist;
-  RF_TILE_LOOP(pdl_wait(), nTiles + n0) {
-    if (t_ >= n0)
-      face_tile<R, 128, 1>(regs, tiles, nTiles, t_ - n0, dist);
-    else if (t_ >= x.dt)
-      bface_tile<R>(regs, x.bface, t_ - x.dt);
-    else
-      dt_finalize_block<R>(regs, x.nRegions, x.coupled, x.a, smin);
-  }
+  flux_merged_body<R>(regs, tiles, nTiles, pfDist, x, smin);
 }
 
 template <typename R>
@@ -3182,7 +3179,6 @@ void launch_stage(const RegionDev<R> *regs, const Work &w, const StepArgs &a, cu
     if (launches) *launches += 1;
     return;
   }
-  auto gsz = [&](int nt) { return w.grid > 0 && w.grid < nt ? w.grid : nt; };
   long long n = 0;
   const bool hasGrad = spaceOrder > 1 && w.nCellTiles > 0;
   const bool grad = hasGrad && (parts & SP_GRADIENT);
