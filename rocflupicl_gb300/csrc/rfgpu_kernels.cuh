@@ -656,7 +656,9 @@ __device__ __forceinline__ void prefetch_ahead(int t, int nTiles, int dist, PF p
 // predecessor writes, for the predecessor's completion; a kernel completes
 // after its own wait, so the order is transitive.  Returns the block's index
 // through the wait, so that every address computed from it (tile, region,
-// cell) is known only afterwards and no load can move ahead.  Measured, a
+// cell) is known only afterwards; what a kernel reads at fixed addresses (the
+// time step's scalars) it reads behind a branch on that index.  So no load can
+// move ahead.  Measured, a
 // residual of 512 cells 41.6 -> 35.3 us, a step of 10,000 tets 73.8 -> 70.8 us.
 // Letting the successor's blocks in earlier (launch_dependents at the start)
 // places them on SMs that are still busy: the 4,000-cell FP64 tube's step 131
@@ -2815,8 +2817,7 @@ template <typename R>
 __global__ void __launch_bounds__(128) k_dt_finalize(const RegionDev<R> *__restrict__ regs,
                                                      int nRegions, int coupled, DtArgs a) {
   __shared__ unsigned long long smin[32];
-  pdl_wait();
-  dt_finalize_block<R>(regs, nRegions, coupled, a, smin);
+  if (pdl_wait() == 0) dt_finalize_block<R>(regs, nRegions, coupled, a, smin);
 }
 template <typename R>
 void launch_dt_finalize(const RegionDev<R> *regs, const Work &w, const DtArgs &a,
