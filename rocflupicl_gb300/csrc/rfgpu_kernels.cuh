@@ -2197,14 +2197,17 @@ __device__ __forceinline__ unsigned after_update(double gc, double gg, double q[
   return st;
 }
 
-// Whether after_update can change a cell or set a bit, apart from NaN
-// velocities and temperatures: not when density, pressure and energy are
-// positive and the pressure is no cancellation residue.  after_update forms the
-// pressure again in another order of operations, and only beyond 2^-30 of the
-// total energy are both sure to be positive.
+// Whether after_update can change a cell or set a bit: not when density, energy
+// and the EOS pressure p are positive and finite and p is no cancellation
+// residue.  after_update forms the pressure again in another order of
+// operations, and only beyond 2^-30 of the total energy are both sure to be
+// positive.  Nothing is NaN then: an infinite or NaN momentum makes p -infinite
+// or NaN, and finite ones over a normal density give no NaN.  One branch for
+// all four tests: 197,000 tets, split update 35.7 us against 36.2 with a branch
+// each.
 __device__ __forceinline__ bool checks_can_act(const double q[5], double p) {
-  return !positive_bits(q[0]) || !positive_bits(p) || !positive_bits(q[4]) ||
-         (unsigned)__double2hiint(p) + (30u << 20) < (unsigned)__double2hiint(q[4]);
+  const unsigned e = (unsigned)__double2hiint(q[4]), h = (unsigned)__double2hiint(p);
+  return !(positive_bits(q[0]) & positive_bits(p) & positive_bits(q[4]) & (h + (30u << 20) >= e));
 }
 
 // Error-free transformation of a + b (Knuth's TwoSum); lo collects the
@@ -2514,7 +2517,7 @@ __device__ __forceinline__ void eos_cell64(const Phys &ph, const double q[5], do
 // 1/V.  The FP32 record (rho, u, v, w, p) for the next stage's gathers is
 // rounded from the FP64 values.  AfterUpdateMP's checks
 // (libfloflu/AfterUpdateMP.F90:134-136) run only on cells they can act on
-// (checks_can_act; finite momenta over a normal density give no NaN).
+// (checks_can_act).
 __device__ __forceinline__ void gather_update_split(const RegionDev<float> &g, int c,
                                                     const StepArgs &a) {
   const int N = g.nCells;
@@ -2587,7 +2590,7 @@ __device__ __forceinline__ void gather_update_split(const RegionDev<float> &g, i
   }
   double ir;
   double p = eos_p(ph, q, ir);
-  if (checks_can_act(q, p) || !finite_bits(q[1]) || !finite_bits(q[2]) || !finite_bits(q[3])) {
+  if (checks_can_act(q, p)) {
     double d[3];
     d[0] = p;
     d[1] = p / (q[0] * ph.gvR);
@@ -2681,8 +2684,7 @@ __device__ __forceinline__ void update_tile(const RT &regs, const Tile *__restri
     eos_cell64(ph, q, ir, d[0], vel);
     d[1] = d[0] / (q[0] * gc);
     d[2] = sqrt(gg * gc * d[1]);
-    if (checks_can_act(q, d[0]) || nan_bits(d[1]) || nan_bits(vel[0]) || nan_bits(vel[1]) ||
-        nan_bits(vel[2])) {
+    if (checks_can_act(q, d[0])) {
       const unsigned st = after_update(gc, gg, q, d);
       if (st) atomicOr(g.status, st);
     }
