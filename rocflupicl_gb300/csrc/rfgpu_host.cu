@@ -146,11 +146,15 @@ struct rfgpu_region_s {
        *phBface = nullptr;
   int phOff[5][9] = {};
   int phN = 0;
-  // mixed-path transfers: the device cells of each chunk in ascending device
-  // order (xList[xOff[k] .. xOff[k+1])), so the conversions touch the device
-  // state coalesced
-  int *xList = nullptr;
-  int xOff[9] = {};
+  // mixed-path transfers: the device cells of each of nk chunks in ascending
+  // device order (list[off[k] .. off[k+1])), so the conversions touch the
+  // device state coalesced; the host-resident step and the plain transfers
+  // share one set where their chunk counts agree
+  struct Chunks {
+    int nk = 0;
+    int *list = nullptr;
+    int off[9] = {};
+  } xc[2];
   // rfgpu_step_host: the upload's conversions run on their own stream, beside
   // the first stage's gradient phases on the region's stream
   cudaStream_t cstream = nullptr;
@@ -846,22 +850,21 @@ void chunk_range(const rfgpu_region_s *h, int k, int nk, int &t0, int &t1, size_
 }
 
 // Chunks of a transfer.  A chunk costs a copy, two events and a launch or two
-// whatever its size, so they hold 131,072 cells or more on average, and two
-// million cells or more make the full 8.  Against 8 chunks for
-// every region: host-resident step of 10,000 cells 295 -> 112 us, 48,000 349 ->
-// 146, 280,000 604 -> 459; upload of 10,000 cells 54 -> 20 us.  6 chunks for
-// 1.57 M cells: 1.72 ms against 1.78 with 8; the same at 3.07 M.
-int n_chunks(const rfgpu_region_s *h) {
-  const int most = h->nCells < (1 << 21) ? 6 : kXChunks;
+// whatever its size, so they hold 131,072 cells or more on average.  Against 8
+// chunks for every region: host-resident step of 10,000 cells 295 -> 112 us,
+// 48,000 349 -> 146, 280,000 604 -> 459; upload of 10,000 cells 54 -> 20 us.
+// The host-resident step, whose stages run by chunk too, takes 6 up to two
+// million cells: 1.57 M cells 1.70 ms against 1.76 with 8, 1.97 M 2.16 against
+// 2.22.  Plain transfers take 8, whose first and last are short: downloads of
+// 1.97 M cells 711 us against 721 with 6.
+int n_chunks(const rfgpu_region_s *h, bool step) {
+  const int most = step && h->nCells < (1 << 21) ? 6 : kXChunks;
   return std::min(most, std::max(1, h->nCells >> 17));
 }
 
-// The second stream, the events and the per-chunk device cell lists of the
-// chunked transfers, made on first use.
-int transfer_setup(rfgpu_region_s *h) {
-  if (h->xstream) return RFGPU_OK;
+// The chunks' device cell lists, made on first use; nk chunks.
+int chunk_lists(rfgpu_region_s *h, int nk, rfgpu_region_s::Chunks &xc) {
   const int N = h->nCells;
-  const int nk = n_chunks(h);
   std::vector<int> old(N), chunk(N), list(N);
   if (h->cellOld) {
     if (cudaMemcpyAsync(old.data(), h->cellOld, (size_t)N * 4, cudaMemcpyDeviceToHost,
@@ -880,14 +883,29 @@ int transfer_setup(rfgpu_region_s *h) {
   }
   for (int d = 0; d < N; ++d) cnt[chunk[old[d]] + 1]++;
   for (int k = 0; k < nk; ++k) cnt[k + 1] += cnt[k];
-  for (int k = 0; k <= nk; ++k) h->xOff[k] = cnt[k];
+  for (int k = 0; k <= nk; ++k) xc.off[k] = cnt[k];
   for (int d = 0; d < N; ++d) list[cnt[chunk[old[d]]]++] = d;
   try {
-    h->xList = h->mem.upload(list, h->stream);
+    xc.list = h->mem.upload(list, h->stream);
   } catch (const std::bad_alloc &) {
     return RFGPU_ERR_NOMEM;
   }
   if (cudaStreamSynchronize(h->stream) != cudaSuccess) return RFGPU_ERR_CUDA;
+  xc.nk = nk;
+  return RFGPU_OK;
+}
+
+// The second stream, the events and the chunks of the chunked transfers (step:
+// of the host-resident step), made on first use.
+int transfer_setup(rfgpu_region_s *h, bool step, const rfgpu_region_s::Chunks *&xc) {
+  const int nk = n_chunks(h, step);
+  rfgpu_region_s::Chunks &c = h->xc[0].nk == 0 || h->xc[0].nk == nk ? h->xc[0] : h->xc[1];
+  if (c.nk == 0) {
+    const int rc = chunk_lists(h, nk, c);
+    if (rc != RFGPU_OK) return rc;
+  }
+  xc = &c;
+  if (h->xstream) return RFGPU_OK;
   // conversions run on a stream of the highest priority, so their blocks go
   // before the stage kernels they run beside
   int loPrio = 0, hiPrio = 0;
@@ -903,17 +921,16 @@ int transfer_setup(rfgpu_region_s *h) {
 }
 
 // Conversions of chunk k between the staged Fortran images and the device state.
-void upload_chunk(rfgpu_region_s *h, int k, const double *cvS, const double *dvS,
-                  cudaStream_t s) {
-  launch_upload_list<float>(regs_of<float>(h), h->xList + h->xOff[k], h->xOff[k + 1] - h->xOff[k],
-                            cvS, dvS, h->prec == RFGPU_PREC_SPLIT, s);
+void upload_chunk(rfgpu_region_s *h, const rfgpu_region_s::Chunks &xc, int k, const double *cvS,
+                  const double *dvS, cudaStream_t s) {
+  launch_upload_list<float>(regs_of<float>(h), xc.list + xc.off[k], xc.off[k + 1] - xc.off[k], cvS,
+                            dvS, h->prec == RFGPU_PREC_SPLIT, s);
   h->launches++;
 }
-void download_chunk(rfgpu_region_s *h, int k, double *cvS, double *dvS,
-                    cudaStream_t st = nullptr) {
-  launch_download_list<float>(regs_of<float>(h), h->xList + h->xOff[k],
-                              h->xOff[k + 1] - h->xOff[k], cvS, dvS,
-                              h->prec == RFGPU_PREC_SPLIT, st ? st : h->stream);
+void download_chunk(rfgpu_region_s *h, const rfgpu_region_s::Chunks &xc, int k, double *cvS,
+                    double *dvS, cudaStream_t st) {
+  launch_download_list<float>(regs_of<float>(h), xc.list + xc.off[k], xc.off[k + 1] - xc.off[k],
+                              cvS, dvS, h->prec == RFGPU_PREC_SPLIT, st);
   h->launches++;
 }
 
@@ -921,14 +938,15 @@ int upload_state(rfgpu_region_s *h, const double *cv, const double *dv) {
   cudaStream_t s = h->stream;
   const int N = h->nCells;
   if (h->prec) {  // mixed: DMA copies into the staging buffers, fused conversion, chunk by chunk
-    int rc = transfer_setup(h);
+    const rfgpu_region_s::Chunks *xc;
+    int rc = transfer_setup(h, false, xc);
     if (rc != RFGPU_OK) return rc;
     cudaStream_t x = h->xstream;
     // the copies start after the work already queued on the region's stream
     if (cudaEventRecord(h->xev[kXChunks], s) != cudaSuccess ||
         cudaStreamWaitEvent(x, h->xev[kXChunks], 0) != cudaSuccess)
       return RFGPU_ERR_CUDA;
-    const int nk = n_chunks(h);
+    const int nk = xc->nk;
     for (int k = 0; k < nk; ++k) {
       int t0, t1;
       size_t c0, c1;
@@ -943,7 +961,7 @@ int upload_state(rfgpu_region_s *h, const double *cv, const double *dv) {
       if (cudaEventRecord(h->xev[k], x) != cudaSuccess ||
           cudaStreamWaitEvent(s, h->xev[k], 0) != cudaSuccess)
         return RFGPU_ERR_CUDA;
-      upload_chunk(h, k, h->stage, dv ? h->stage2 : nullptr, s);
+      upload_chunk(h, *xc, k, h->stage, dv ? h->stage2 : nullptr, s);
     }
     return cuda_rc(cudaGetLastError());
   }
@@ -970,7 +988,7 @@ int phase_setup(rfgpu_region_s *h) {
   if (h->phN) return RFGPU_OK;
   const Work &w = h->work;
   const int nT = w.nCellTiles;
-  const int nk = n_chunks(h);
+  const int nk = n_chunks(h, true);
   ChunkMap m{};
   m.nk = nk;
   m.block = w.block;
@@ -1099,7 +1117,8 @@ int phase_setup(rfgpu_region_s *h) {
 // rfgpu_download.  Second order only (the stage-1 gradient pass carries the
 // time step).
 int step_host_mixed(rfgpu_region_s *h, double *cv, double *dv, const DtArgs &da) {
-  int rc = transfer_setup(h);
+  const rfgpu_region_s::Chunks *xc;
+  int rc = transfer_setup(h, true, xc);
   if (rc != RFGPU_OK) return rc;
   rc = phase_setup(h);
   if (rc != RFGPU_OK) return rc;
@@ -1126,7 +1145,7 @@ int step_host_mixed(rfgpu_region_s *h, double *cv, double *dv, const DtArgs &da)
         cudaEventRecord(h->xev[k], x) != cudaSuccess ||
         cudaStreamWaitEvent(cs, h->xev[k], 0) != cudaSuccess)
       return RFGPU_ERR_CUDA;
-    upload_chunk(h, k, h->stage, nullptr, cs);
+    upload_chunk(h, *xc, k, h->stage, nullptr, cs);
     if (cudaEventRecord(h->cev[k], cs) != cudaSuccess ||
         cudaStreamWaitEvent(s, h->cev[k], 0) != cudaSuccess)
       return RFGPU_ERR_CUDA;
@@ -1181,7 +1200,7 @@ int step_host_mixed(rfgpu_region_s *h, double *cv, double *dv, const DtArgs &da)
       if (cudaEventRecord(h->cev[k], s) != cudaSuccess ||
           cudaStreamWaitEvent(cs, h->cev[k], 0) != cudaSuccess)
         return RFGPU_ERR_CUDA;
-      download_chunk(h, k, h->stage, dv ? h->stage2 : nullptr, cs);
+      download_chunk(h, *xc, k, h->stage, dv ? h->stage2 : nullptr, cs);
       if (cudaEventRecord(h->xev[k], cs) != cudaSuccess ||
           cudaStreamWaitEvent(x, h->xev[k], 0) != cudaSuccess)
         return RFGPU_ERR_CUDA;
@@ -1501,16 +1520,17 @@ int rfgpu_download(rfgpu_region_t h, double *cv, double *dv) {
   const int N = h->nCells;
   if (h->prec) {  // mixed: fused conversion into the staging buffers and DMA copies, chunk by chunk
     if (!cv && !dv) return RFGPU_OK;
-    int rc = transfer_setup(h);
+    const rfgpu_region_s::Chunks *xc;
+    int rc = transfer_setup(h, false, xc);
     if (rc != RFGPU_OK) return rc;
     cudaStream_t x = h->xstream;
-    const int nk = n_chunks(h);
+    const int nk = xc->nk;
     for (int k = 0; k < nk; ++k) {
       int t0, t1;
       size_t c0, c1;
       chunk_range(h, k, nk, t0, t1, c0, c1);
       if (t1 <= t0) continue;
-      download_chunk(h, k, cv ? h->stage : nullptr, dv ? h->stage2 : nullptr);
+      download_chunk(h, *xc, k, cv ? h->stage : nullptr, dv ? h->stage2 : nullptr, h->stream);
       if (cudaEventRecord(h->xev[k], h->stream) != cudaSuccess ||
           cudaStreamWaitEvent(x, h->xev[k], 0) != cudaSuccess)
         return RFGPU_ERR_CUDA;

@@ -33,7 +33,8 @@ def box(dims):
 
 @pytest.mark.parametrize("chunks,dims", [
     (1, (44, 35, 28)), (2, (44, 35, 29)), (3, (41, 41, 40)), (4, (45, 45, 44)),
-    (5, (48, 48, 48)), (6, (51, 51, 51)), (8, (71, 71, 70))])
+    (5, (48, 48, 48)), (6, (51, 51, 51)), (8, (71, 71, 70)),
+    (7, (54, 54, 54)), (8, (59, 59, 59))])   # here the step itself runs in 6
 @pytest.mark.parametrize("order", [E.ORDER_HOST, E.ORDER_LOCALITY])
 @pytest.mark.parametrize("variant", sorted(VARIANTS))
 def test_phased_step_equals_three_calls(chunks, dims, order, variant):
