@@ -2968,11 +2968,21 @@ void face_launch(const RegionDev<R> *regs, const Work &w, const Tile *tiles, int
   }
 }
 
-// The merged launch is never the slower one beyond 0.1% (ms per step, separate
-// -> merged: 512 cells 0.0457 -> 0.0353 a residual, 4,000-cell tube FP64 0.166
-// -> 0.131, 10,000 tets 0.082 -> 0.071, 197,000 tets 0.330 -> 0.313, 6.75 M tets
-// 4.571 -> 4.547, split 6.130 -> 6.075, 12.6 M tets 8.099 -> 8.072, split
-// 11.04 -> 10.95; FP64 8.4 M tets 81.52 -> 81.59).
+// The merged launch pays for single regions of every size (ms per step,
+// separate -> merged: 512 cells 0.0457 -> 0.0353 a residual, 4,000-cell tube
+// FP64 0.166 -> 0.131, 10,000 tets 0.082 -> 0.071, 197,000 tets 0.330 -> 0.313,
+// 6.75 M tets 4.571 -> 4.547, split 6.130 -> 6.075, 12.6 M tets 8.099 -> 8.072,
+// split 11.04 -> 10.95; FP64 8.4 M tets 81.52 -> 81.59, no difference) and for
+// FP64 batches (1,500 face tiles 0.726 -> 0.687, 35,000 12.79 -> 12.71).  The
+// FP32-flux kernel over a batch's table holds more registers, which costs large
+// batches more than a launch: 35,000 tiles 1.635 -> 1.626, split 2.432 -> 2.424,
+// but 71,000 tiles 3.127 -> 3.133, split 4.728 -> 4.744, and 314,000 tiles 14.37
+// -> 14.69.
+constexpr int kMergeBatchTiles = 50000;
+template <typename R>
+bool merge_pays(const Work &w) {
+  return w.one || sizeof(R) == 8 || w.nFaceTiles < kMergeBatchTiles;
+}
 template <typename R>
 void merged_launch(const RegionDev<R> *regs, const Work &w, FluxExtra x, cudaStream_t s) {
   const int grid = grid_for(w.grid, w.nFaceTiles + x.nBFace + x.dt);
@@ -3203,7 +3213,7 @@ void launch_stage(const RegionDev<R> *regs, const Work &w, const StepArgs &a, cu
   const bool dt = a.fuseDt && hasGrad && flux, bface = flux && w.nBFaceTiles > 0;
   const bool faces = flux && !(parts & SP_NOFACE) && w.nFaceTiles > 0;
   const bool tuned = w.faceBlock != 0 && (w.faceBlock != 128 || w.facesPerThread != 1);
-  const bool merge = faces && !prof && !tuned && (dt || bface);
+  const bool merge = faces && !prof && !tuned && (dt || bface) && merge_pays<R>(w);
   if (dt && !merge) {
     RF_MARK(KP_DT_FINAL, 0);
     launch_dt_finalize<R>(regs, w, a.dt, s);
