@@ -247,18 +247,17 @@ long long rfgpu_device_bytes(rfgpu_region_t h);
 long long rfgpu_launch_count(rfgpu_region_t h);
 /* Launch shapes of the stage passes, chosen by the autotuner
  * (rocflupicl_gb300/autotune.py) by timing real steps.  The default shapes
- * have launches that others give up: a gradBlock, faceBlock, facesPerThread or
+ * have launches that others give up.  A gradBlock, faceBlock, facesPerThread or
  * cellBlock other than the default makes its pass read the region's descriptor
  * from memory instead of its launch parameters (on the FP64 path cellBlock's
- * alone), a
- * faceBlock or facesPerThread other than the default also launches interior
- * faces, boundary faces and the time step's finalisation one by one, and a
- * gradBlock or gridCap other than the default forgoes the gradient pass for
- * regions of at most 51,072 cells (reduced-precision paths).  Block sizes, faces per
- * thread and the grid leave every result bit for bit unchanged; the persistent
- * stage does on the FP64 path, and on the reduced-precision paths changes
- * results by FP32 rounding at most (the compiler may contract a product into
- * an FMA differently inside the one large kernel).  A zero field keeps the
+ * alone).  A faceBlock or facesPerThread other than the default also launches
+ * interior faces, boundary faces and the time step's finalisation one by one.
+ * A gradBlock or gridCap other than the default forgoes the gradient kernel of
+ * small regions (at most 51,072 cells, reduced-precision paths).  Block sizes,
+ * faces per thread and the grid leave every result bit for bit unchanged; the
+ * persistent stage does on the FP64 path, and on the reduced-precision paths
+ * changes results by FP32 rounding at most (the compiler may contract a product
+ * into an FMA differently inside the one large kernel).  A zero field keeps the
  * default.  No counterpart in the reference (its loops run serially on the
  * host). */
 typedef struct {
