@@ -288,10 +288,10 @@ int rfgpu_set_tuning(rfgpu_region_t h, const rfgpu_tuning_t *t);
 /* Per-kernel profiler (the engine's counterpart of the reference's ROCPROF
  * FPROFILER_BEGINS/ENDS markers): while enabled, CUDA events are recorded on
  * the handle's stream around every kernel, and the flux passes of a stage,
- * otherwise one launch, are launched one by one: the times are the passes'
- * own, their sum more than an unprofiled step; rfgpu_profile_read synchronises and
- * returns, per kernel class, the summed milliseconds and launch counts, then
- * resets.  Classes: 0 gradient, 1 limiter, 2 face flux, 3 boundary-face flux,
+ * otherwise one launch (large reduced-precision batches apart), are launched
+ * one by one: the times are the passes' own, their sum more than an unprofiled
+ * step; rfgpu_profile_read synchronises and returns, per kernel class, the
+ * summed milliseconds and launch counts, then resets.  Classes: 0 gradient, 1 limiter, 2 face flux, 3 boundary-face flux,
  * 4 gather+update, 5 dt faces, 6 dt boundary faces, 7 dt cells, 8 dt finalize,
  * 9 halo exchange, 10 a whole stage run as one persistent launch.  Graph
  * replays are not profiled. */
